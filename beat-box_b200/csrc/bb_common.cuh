@@ -19,6 +19,7 @@
 
 #define BB_MAX_CONTACTS 8
 #define BB_MAX_COLORS 32
+#define BB_GC_CLASSES 7u  // contact-count classes of a colour's bucket: (32 + 2) x 7 keys fit one 8-bit digit
 #define BB_UNCOLORED BB_EDGE_COLOR_OVERFLOW
 #define BB_RESTING BB_EDGE_COLOR_RESTING  // a manifold whose island has no awake body (not coloured)
 #define BB_NONE 0xFFFFFFFFu
@@ -137,17 +138,17 @@ struct DevState {
   float4* c_kt[2];       // AVBD tangent penalties 0/1, stick (bits), warm-start count (bits)
   float4* c_anc_a[2];    // AVBD local anchor on a .xyz, feature pair (bits)
   float4* c_anc_b[2];    // AVBD local anchor on b .xyz, 0
-  // PGS rows (current only)
+  // PGS rows (current only).  Colour sweeps: c_r1 = (position, normal mass), c_r2 as float2 =
+  // tangent masses, c_k = the bodies' tagged velocities.
   float4 *c_r1, *c_r2, *c_k;
-  // dataflow schedule: per compact manifold (slot, a, b, rank_a | rank_b << 16); per-body counters
+  // colour sweeps: as float2, y and z of each item's anchor on b; colours of each body's items
   uint4* flow_rec;
   uint32_t* flow_counter;
-  // barrier schedule: colour-ordered items, rec = (slot, a, b, cc | dyn_a << 8 | dyn_b << 9 |
-  // skip << 10), mass = (inverse mass a, inverse mass b, friction, -)
+  // colour sweeps: colour-ordered items (record, anchors, three frame planes), impulses and bias
   uint4* pgs_rec;
   float4* pgs_mass;
-  float4* pgs_frame;   // 3 per item: normal, tangent 0, tangent 1
-  float4* pgs_lam;     // compact impulses, pgs_coff[k] + j
+  float4* pgs_frame;
+  float4* pgs_lam;
   uint32_t *pgs_cnt, *pgs_coff, *pgs_slot;
   // per-body manifold lists (CSR over compact manifold indices) [cur], [prev]
   uint32_t* csr_start[2];
@@ -172,7 +173,7 @@ struct DevState {
   unsigned long long* gc_owner; // 32 colours x (body capacity + 1) bodies: (epoch << 32) | priority
   uint32_t *bucket_keys[2], *bucket_vals[2]; // colour sort of manifolds / bodies
   uint32_t* bucket_start; // 34 + 32*L entries
-  uint32_t* colour_awake; // per colour (32 = overflow): 1 if one of its manifolds has an awake body
+  uint32_t* colour_awake; // not used (kept: the arrays are the layout of saved states)
   // colour reuse: an island whose manifolds (bodies and key) are exactly last substep's keeps
   // last substep's colours (the colouring of an island depends on that set alone)
   uint32_t* gc_slot_color[2]; // per manifold slot of each buffer: the colour the colouring gave it
@@ -343,7 +344,7 @@ __device__ __forceinline__ Sym3 body_world_inv_inertia(const float4* iinv, const
 }
 
 // Sites of bounded waits, recorded in DevCounters::error_site by the first one that gives up
-// (bb_step_stats.error_site): the sort's and the scan's look-backs, the dataflow PGS wait,
+// (bb_step_stats.error_site): the sort's and the scan's look-backs, the PGS_SOFT sweeps' wait for a body,
 // the generation barrier, and BB_SITE_GRID + k for the grid barrier on sync_count[k] (0 edge colouring, 1
 // PGS_SOFT, 2 AVBD colouring, 3..5 AVBD solve phases, 7 connected components).
 #define BB_SITE_SORT 1u

@@ -467,22 +467,24 @@ __global__ void __launch_bounds__(BB_GC_THREADS, 1) k_edge_color(const DevState 
   }
   if (local) grid_sync(c, sync, ep);  // block 0's rounds are done before anyone reads the colours
   if (blockIdx.x == 0 && threadIdx.x == 0) c->gc_rounds_run = ran;
-  // Keys: colour, 32 = overflow, 33 = not swept.  Under the colour-barrier schedule a coloured
-  // manifold whose two bodies are both asleep or static is also keyed 33: its sweep items would
-  // do nothing (both bodies are frozen this substep), and leaving them out of the colour lists
-  // saves the sweeps from walking them.  Its colour (gc_color) is kept.  The dataflow schedule
-  // ranks every manifold on a body's list, so there every coloured manifold stays in its colour.
-  const bool drop_idle = p.schedule == BB_SCHEDULE_COLOUR_BARRIER;
+  // Keys of the bucket sort: colour (32 = overflow, 33 = not swept) x BB_GC_CLASSES + class, the
+  // classes of a colour by falling contact count (the colour-sweep kernel's warps then hold items
+  // of equal length; the items of a colour are independent, so their order is free).  The
+  // overflow bucket is one class: it runs in manifold order.  A coloured manifold whose two bodies are
+  // both asleep or static is also keyed 33: its sweep items would do nothing (both bodies are
+  // frozen this substep).  Its colour (gc_color) is kept.
   uint32_t over = 0;
   for (uint32_t m = tid; m < M; m += stride) {
     uint32_t col = d.gc_color[m];
     if (col == BB_UNCOLORED) ++over;
     uint32_t key = col == BB_UNCOLORED ? BB_MAX_COLORS : col == BB_RESTING ? BB_MAX_COLORS + 1 : col;
-    if (drop_idle && key <= BB_MAX_COLORS && (reinterpret_cast<const uint32_t*>(d.gc_rec + m)[3] & 4u))
-      key = BB_MAX_COLORS + 1;
-    d.bucket_keys[0][m] = key;
+    if (key <= BB_MAX_COLORS && (reinterpret_cast<const uint32_t*>(d.gc_rec + m)[3] & 4u)) key = BB_MAX_COLORS + 1;
+    const uint32_t slot = d.man_slot[cur][m];
+    uint32_t cls = 0;
+    if (key < BB_MAX_COLORS) cls = BB_GC_CLASSES - min(max(uint32_t(d.m_keycc[cur][slot].y), 1u), BB_GC_CLASSES);
+    d.bucket_keys[0][m] = key * BB_GC_CLASSES + cls;
     d.bucket_vals[0][m] = m;
-    d.gc_slot_color[cur][d.man_slot[cur][m]] = col;  // for the next substep's colour reuse
+    d.gc_slot_color[cur][slot] = col;  // for the next substep's colour reuse
   }
   if (over) atomicAdd(&c->gc_overflow, over);
   if (tid == 0) {
@@ -494,7 +496,7 @@ __global__ void __launch_bounds__(BB_GC_THREADS, 1) k_edge_color(const DevState 
 // bucket_start[0..34]: start of colour c (32 = overflow, 33 = resting manifolds), [34] = M
 __global__ void k_bucket_starts(const uint32_t* hist_scan, const uint32_t* n_ptr, uint32_t* starts, int nb) {
   int t = threadIdx.x;
-  if (t < nb) starts[t] = hist_scan[t];
+  if (t < nb) starts[t] = hist_scan[t * int(BB_GC_CLASSES)];
   if (t == nb) starts[t] = *n_ptr;
 }
 

@@ -74,7 +74,7 @@ void bb_sort_carve(char* base, uint32_t n, int passes, DevCounters** ctr, uint32
 
 // co-resident block counts of the persistent cooperative kernels
 int bb_edge_coloring_blocks(int sms);
-int bb_pgs_soft_blocks(int sms);
+int bb_pgs_soft_blocks(int sms, uint32_t max_bodies);
 int bb_avbd_blocks(int sms);
 
 // occupancy helpers (bb_world.cu)

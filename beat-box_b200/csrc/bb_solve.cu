@@ -9,10 +9,10 @@
 // (:132-202), post-stabilisation sweeps (RBM:1400-1425).
 //
 // B200 design: each solver phase is ONE persistent cooperative kernel that walks compact
-// colour buckets and separates colours with a grid barrier, instead of the reference's
-// (2I+1) x 33 dispatches that each scan every manifold and filter by colour.  Contact rows
-// are 64-byte float4 groups per contact; body velocities and the world inverse inertia are
-// float4 loads.  The 6x6 block solve stays in registers.
+// colour buckets, instead of the reference's (2I+1) x 33 dispatches that each scan every
+// manifold and filter by colour.  The PGS_SOFT sweeps order the updates of a body by a tag in its
+// velocity words; the AVBD sweeps separate colours with a grid barrier.  The 6x6 block solve
+// stays in registers.
 #include "bb_common.cuh"
 #include <algorithm>
 
@@ -51,12 +51,10 @@ __device__ __forceinline__ Quatf apply_angular_velocity(Quatf rot, float3 w, flo
   return q_normalize(q_mul(q, rot));
 }
 
-// ---- PGS_SOFT arithmetic of one contact, shared by both schedules (same expressions, so the
-// schedules agree bit for bit) -------------------------------------------------------------
+// ---- PGS_SOFT arithmetic of one contact ---------------------------------------------------
 
 // Every operation below is an explicitly rounded intrinsic (fma where a product feeds a sum),
-// so the compiler has nothing left to contract: each inlined copy of this arithmetic -- the
-// barrier schedule's register-held and streamed contacts, the dataflow schedule -- produces
+// so the compiler has nothing left to contract: each inlined copy of this arithmetic produces
 // the same bits.
 __device__ __forceinline__ float3 xadd(float3 a, float3 b) {
   return make_float3(__fadd_rn(a.x, b.x), __fadd_rn(a.y, b.y), __fadd_rn(a.z, b.z));
@@ -267,14 +265,14 @@ __device__ void pgs_solve_slot(const DevState& d, const Params& p, int cur, uint
 }
 
 // integrate one body (RB_sim.slang:1287-1326) and refresh its world inverse inertia
-// Compiled once (not inlined) so both schedules integrate with the same instructions.
-__device__ __noinline__ void pgs_integrate_body(float4* pos, float4* rot, const float4* vel, const float4* omega,
+// Compiled once (not inlined) so every path integrates with the same instructions.
+__device__ __noinline__ void pgs_integrate_body(float4* pos, float4* rot, float4 vel, float4 omega,
                                                 const float4* iinv, const float4* ioff, bool full, float4* iw,
                                                 uint32_t i, float h, bool tq) {
   const float4 ps = pos[i];
-  const float3 v = f3(vel[i]);
+  const float3 v = f3(vel);
   pos[i] = make_float4(ps.x + v.x * h, ps.y + v.y * h, ps.z + v.z * h, ps.w);
-  const Quatf q = apply_angular_velocity(q_from(rot[i]), f3(omega[i]), h);
+  const Quatf q = apply_angular_velocity(q_from(rot[i]), f3(omega), h);
   rot[i] = q_to4(q);
   const Sym3 s = body_world_inv_inertia(iinv, ioff, full, i, q, tq);
   iw[2 * i] = make_float4(s.xx, s.xy, s.xz, s.yy);
@@ -290,617 +288,519 @@ __device__ __forceinline__ void pgs_world_inertia(const DevState& d, uint32_t i,
   pgs_world_inertia_body(d.rot, d.iinv, d.iinv_off, d.full_inertia != 0, d.iw, i, tq);
 }
 __device__ __forceinline__ void pgs_integrate(const DevState& d, uint32_t i, float h, bool tq) {
-  pgs_integrate_body(d.pos, d.rot, d.vel, d.omega, d.iinv, d.iinv_off, d.full_inertia != 0, d.iw, i, h, tq);
+  pgs_integrate_body(d.pos, d.rot, d.vel[i], d.omega[i], d.iinv, d.iinv_off, d.full_inertia != 0, d.iw, i, h, tq);
 }
 
 // ---------------------------------------------------------------------------------------
-// PGS_SOFT, colour-barrier schedule: one persistent cooperative kernel.
+// PGS_SOFT on colours: one persistent cooperative kernel without a barrier between colours.
 //
-// Every sweep walks the colour buckets in order with a grid barrier after each colour; item k
-// of a colour (a manifold) always belongs to the same thread, so the thread can load the
-// next colour's item -- its record, contact frame, rows and impulses, none of which another
-// thread writes -- BEFORE the barrier, and after the barrier only the two bodies' velocities
-// and inertias remain to be fetched: one memory round trip per colour on the critical path.
-#define BB_PGS_THREADS 256  // one block per SM: up to 255 registers for the held item
-#define BB_PGS_SKIP (1u << 10)
+// The sweeps give every body the ordered sequence of its manifolds by colour, and a manifold's
+// result depends only on its two bodies' velocities.  So each body's velocity carries a tag: the
+// number of updates it has had.  An item (a manifold) of sweep s waits until its two bodies
+// carry s * degree + rank (the body's swept manifolds, and the item's place among them), runs,
+// and stores them with the tag one higher.  Velocity and tag share one 16-byte word, loaded
+// and stored as one (b128, relaxed, gpu scope), so a wait is the load of the data itself: no
+// barrier, no fence and no separate flag.  The same order on every body as one barrier per
+// colour gives, hence the same bits.
+//
+// Items are taken 32 at a time, a tile: a warp's lanes, all of one colour, so none waits for
+// another lane of its warp.  Warp w of W runs the tiles w, w + W, ... in (sweep, colour)
+// order, every wait points at an earlier tile, and all blocks are resident: no deadlock.
+// Within a colour the items are sorted by contact count, so a tile's lanes run equally long.
+//
+// Layout: a compact copy in colour order.  Per item 88 bytes in planes of float4 (a warp reads
+// 512 consecutive bytes), per contact 40 bytes: (position, normal mass), (tangent masses),
+// (impulses, bias).  Contact j of a tile's lanes is stored lane after lane (those that have a
+// contact j), after contact j - 1 of all: dense, and one run per load.  The lever arms are
+// the contact's position minus the two anchors, as the pre-step forms them.
+#define BB_PGS_THREADS 64
+#define BB_PGS_PER_SM 4
+#define BB_PGS_CLASSES BB_GC_CLASSES
+#define BB_PGS_PF 4  // contacts of an item loaded together
 
-// The kernel works on a compact copy in colour order: item k's record, masses and contact frame
-// at index k, its contacts' rows (c_r1, c_r2, c_k reused with compact indexing) and impulses
-// (pgs_lam) at pgs_coff[k] + j.  The impulses go back to the persistent slot-indexed contacts
-// when the kernel ends.  Dense arrays keep the per-sweep working set (about 80 B per manifold,
-// 64 B per contact, 64 B per body) resident in L2.
-template <int PF>  // contacts of an item held in registers across the barrier
-struct PgsItem {
-  uint4 rec;    // contact offset, body a, body b, contact count | dynamic a << 8 | dynamic b << 9 | skip << 10
-  float4 mass;  // inverse mass a, inverse mass b, friction, -
-  float4 n, t0, t1;
-  float4 R1[PF], R2[PF], K[PF], lam[PF];
+// body i's tagged velocities (linear, angular) next to each other, in row scratch this solver
+// does not use
+__device__ __forceinline__ float4* pgs_vw(const DevState& d) { return d.c_k; }
+__device__ __forceinline__ float2* pgs_tmass(const DevState& d) { return reinterpret_cast<float2*>(d.c_r2); }
+__device__ __forceinline__ float2* pgs_anchor(const DevState& d) { return reinterpret_cast<float2*>(d.flow_rec); }
+
+__device__ __forceinline__ float4 ld_tagged(const float4* p) {
+  unsigned long long lo, hi;
+  asm volatile("{\n\t.reg .b128 t;\n\tld.relaxed.gpu.global.b128 t, [%2];\n\tmov.b128 {%0, %1}, t;\n\t}"
+               : "=l"(lo), "=l"(hi)
+               : "l"(p)
+               : "memory");
+  return make_float4(__uint_as_float(uint32_t(lo)), __uint_as_float(uint32_t(lo >> 32)), __uint_as_float(uint32_t(hi)),
+                     __uint_as_float(uint32_t(hi >> 32)));
+}
+__device__ __forceinline__ void st_tagged(float4* p, float3 v, uint32_t tag) {
+  const unsigned long long lo = (unsigned long long)__float_as_uint(v.x) | ((unsigned long long)__float_as_uint(v.y) << 32);
+  const unsigned long long hi = (unsigned long long)__float_as_uint(v.z) | ((unsigned long long)tag << 32);
+  asm volatile("{\n\t.reg .b128 t;\n\tmov.b128 t, {%1, %2};\n\tst.relaxed.gpu.global.b128 [%0], t;\n\t}"
+               :
+               : "l"(p), "l"(lo), "l"(hi)
+               : "memory");
+}
+
+// tiles of the colour lists: first tile of each colour (from the colour count on: the number of
+// tiles) and first item of each colour
+struct PgsTiles {
+  uint32_t first[BB_MAX_COLORS + 1];
+  uint32_t start[BB_MAX_COLORS + 2];
 };
-
-// Contacts beyond the PF register-held ones (up to BB_MAX_CONTACTS - PF) are staged in this
-// thread's slot of dynamic shared memory with cp.async at prefetch time, so the run does not
-// pay one global round trip per extra contact.  Slot layout: [contact][R1, R2, K, lam].
-#define BB_PGS_EXTRA (BB_MAX_CONTACTS - 4)
-// Next-item staging (k_pgs_soft): the item a thread runs after the current one in the same
-// colour -- masses, frame, up to four contacts' rows and impulses, and both bodies' velocities
-// and world inverse inertias -- copied with cp.async while the current item computes.  Element e
-// of thread t sits at e * BB_PGS_THREADS + t, so a warp's 16-byte accesses hit distinct banks.
-#define BB_PGS_NEXT 28  // float4 per thread: mass, n, t0, t1, 4 x (R1, R2, K, lam), 8 body words
-#define BB_PGS_SMEM_EXTRA (BB_PGS_THREADS * BB_PGS_EXTRA * 4 * 16)
-#define BB_PGS_SMEM (BB_PGS_SMEM_EXTRA + BB_PGS_THREADS * BB_PGS_NEXT * 16)
-__device__ __forceinline__ float4* pgs_extra_slot() {
-  extern __shared__ float4 s_pgs_extra[];
-  return s_pgs_extra + threadIdx.x * (BB_PGS_EXTRA * 4);
-}
-__device__ __forceinline__ float4* pgs_next_base() {
-  extern __shared__ float4 s_pgs_extra[];
-  return s_pgs_extra + BB_PGS_THREADS * BB_PGS_EXTRA * 4 + threadIdx.x;
-}
-__device__ __forceinline__ void cp_async16(void* smem, const void* gmem) {
-  const uint32_t s = uint32_t(__cvta_generic_to_shared(smem));
-  asm volatile("cp.async.ca.shared.global [%0], [%1], 16;" ::"r"(s), "l"(gmem) : "memory");
-}
-__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
-__device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_all;" ::: "memory"); }
-
-// STAGED: extra contacts go to shared memory (the persistent kernels); else they stay in global
-// memory and the run reads them there (the serial overflow path, which must not disturb the
-// slot of the item already prefetched for the next colour).
-template <int PF, bool STAGED>
-__device__ __forceinline__ void pgs_item_fill(const DevState& d, uint32_t k, PgsItem<PF>& x) {
-  x.mass = d.pgs_mass[k];
-  x.n = d.pgs_frame[3 * k];
-  x.t0 = d.pgs_frame[3 * k + 1];
-  x.t1 = d.pgs_frame[3 * k + 2];
-  const uint32_t c0 = x.rec.x, cc = x.rec.w & 0xFFu;
+__device__ __forceinline__ void pgs_tiles(const DevState& d, PgsTiles& ft) {
+  if (threadIdx.x < 32u) {
+    const uint32_t lane = threadIdx.x;
+    const uint32_t s0 = d.bucket_start[lane], s1 = d.bucket_start[lane + 1];
+    uint32_t v = lane < d.ctr->gc_colors ? (s1 - s0 + 31u) / 32u : 0u;
+    const uint32_t own = v;
 #pragma unroll
-  for (int j = 0; j < PF; ++j) {
-    if (uint32_t(j) < cc) {
-      x.R1[j] = d.c_r1[c0 + j];
-      x.R2[j] = d.c_r2[c0 + j];
-      x.K[j] = d.c_k[c0 + j];
-      x.lam[j] = d.pgs_lam[c0 + j];
+    for (int o = 1; o < 32; o <<= 1) {
+      const uint32_t u = __shfl_up_sync(0xFFFFFFFFu, v, o);
+      if (int(lane) >= o) v += u;
+    }
+    ft.first[lane] = v - own;
+    ft.start[lane] = s0;
+    if (lane == 31u) {
+      ft.first[32] = v;
+      ft.start[32] = s1;
+      ft.start[33] = d.bucket_start[BB_MAX_COLORS + 1];
     }
   }
-  if (STAGED && cc > uint32_t(PF)) {
-    float4* slot = pgs_extra_slot();
-    for (uint32_t j = PF; j < cc; ++j) {
-      float4* e = slot + (j - PF) * 4;
-      cp_async16(e + 0, d.c_r1 + c0 + j);
-      cp_async16(e + 1, d.c_r2 + c0 + j);
-      cp_async16(e + 2, d.c_k + c0 + j);
-      cp_async16(e + 3, d.pgs_lam + c0 + j);
-    }
-    cp_async_commit();
+  __syncthreads();
+}
+// item of this lane in tile t (BB_NONE past the colour's end)
+__device__ __forceinline__ uint32_t pgs_tile_item(const PgsTiles& ft, uint32_t t) {
+  const uint32_t lane = threadIdx.x & 31u;
+  const uint32_t c = uint32_t(__popc(__ballot_sync(0xFFFFFFFFu, ft.first[lane] <= t))) - 1u;
+  const uint32_t k = ft.start[c] + (t - ft.first[c]) * 32u + lane;
+  return k < ft.start[c + 1] ? k : BB_NONE;
+}
+
+// item record: x, y: bodies, bit 31 = dynamic; z: contact count | rank on a << 4 | degree of a
+// << 9 | rank on b << 15 | degree of b << 20; w: first contact of the item's tile (overflow:
+// of the item)
+#define PGS_BODY(x) ((x) & 0x7FFFFFFFu)
+
+// before the sweeps, per body: world inverse inertia, tagged velocities, no colours yet
+__global__ void k_pgs_bodies(const DevState d, uint32_t n, Params p) {
+  const bool tq = p.quirks & BB_QUIRK_INERTIA_TRANSPOSE;
+  float4* vw = pgs_vw(d);
+  for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+    pgs_world_inertia(d, i, tq);
+    d.flow_counter[i] = 0u;
+    vw[2 * size_t(i)] = f4(f3(d.vel[i]), 0.f);
+    vw[2 * size_t(i) + 1] = f4(f3(d.omega[i]), 0.f);
   }
 }
 
-// item k given its record (loaded ahead): masses, frame, rows, impulses
-template <int PF, bool STAGED = true>
-__device__ __forceinline__ void pgs_item_load_rest(const DevState& d, uint32_t k, uint4 rec, PgsItem<PF>& x) {
-  x.rec = rec;
-  pgs_item_fill<PF, STAGED>(d, k, x);
-}
-
-template <int PF, bool STAGED = true>
-__device__ __forceinline__ void pgs_item_load(const DevState& d, uint32_t k, PgsItem<PF>& x) {
-  x.rec = d.pgs_rec[k];
-  pgs_item_fill<PF, STAGED>(d, k, x);
-}
-
-// contacts per colour-ordered item (0 for items whose bodies both sleep): scanned into pgs_coff
+// per swept item (colours and overflow): contact count, to be scanned; its colour in the masks of
+// its dynamic bodies (a body's rank and degree are bit counts of its mask)
 __global__ void k_pgs_count(const DevState d, int cur) {
-  const uint32_t M = d.ctr->manifold_count;
+  const uint32_t end = d.bucket_start[BB_MAX_COLORS + 1], over = d.bucket_start[BB_MAX_COLORS];
   const uint32_t* list = d.bucket_vals[1];
-  for (uint32_t k = blockIdx.x * blockDim.x + threadIdx.x; k < M; k += gridDim.x * blockDim.x) {
-    const uint32_t slot = d.man_slot[cur][list[k]];
+  if (blockIdx.x == 0 && threadIdx.x == 0) d.ctr->pgs_manifolds = end;
+  for (uint32_t k = blockIdx.x * blockDim.x + threadIdx.x; k < end; k += gridDim.x * blockDim.x) {
+    const uint32_t m = list[k], slot = d.man_slot[cur][m];
+    d.pgs_slot[k] = slot;
+    d.pgs_cnt[k] = uint32_t(d.m_keycc[cur][slot].y);
+    if (k >= over) continue;
     const uint2 b = d.m_bodies[cur][slot];
-    const bool skip = !awake(d.flags[b.x]) && !awake(d.flags[b.y]);
-    d.pgs_cnt[k] = skip ? 0u : uint32_t(d.m_keycc[cur][slot].y);
-    const uint32_t act = __ballot_sync(__activemask(), !skip);
-    if ((threadIdx.x & 31u) == uint32_t(__ffs(__activemask()) - 1) && act) atomicAdd(&d.ctr->pgs_manifolds, __popc(act));
-    if (!skip) {  // set once: most threads only read the flag (33 hot words otherwise take every store)
-      uint32_t* f = &d.colour_awake[min(d.gc_color[list[k]], uint32_t(BB_MAX_COLORS))];
-      if (*f == 0u) *f = 1u;
-    }
+    const uint32_t bit = 1u << d.gc_color[m];
+    if (d.flags[b.x] & BB_BODY_DYNAMIC) atomicOr(&d.flow_counter[b.x], bit);
+    if (d.flags[b.y] & BB_BODY_DYNAMIC) atomicOr(&d.flow_counter[b.y], bit);
   }
 }
 
-// compact record + rows of colour-ordered item k (the pre-step's row half; no body is touched)
-__device__ void pgs_item_build(const DevState& d, int cur, uint32_t k, uint32_t m, float h, float hertz) {
-  const uint32_t slot = d.man_slot[cur][m];
-  const uint2 b = d.m_bodies[cur][slot];
-  const uint32_t fa = d.flags[b.x], fb = d.flags[b.y];
-  const uint32_t cc = d.pgs_cnt[k];  // 0 when both bodies sleep
-  const uint32_t c0 = d.pgs_coff[k];
-  const bool skip = !awake(fa) && !awake(fb);
-  const float ima = d.pos[b.x].w, imb = d.pos[b.y].w;
-  d.pgs_rec[k] = make_uint4(c0, b.x, b.y,
-                            cc | ((fa & BB_BODY_DYNAMIC) ? 1u << 8 : 0u) | ((fb & BB_BODY_DYNAMIC) ? 1u << 9 : 0u) |
-                                (skip ? BB_PGS_SKIP : 0u));
-  d.pgs_mass[k] = make_float4(ima, imb, sqrtf(d.iinv[b.x].w * d.iinv[b.y].w), 0.f);
-  d.pgs_slot[k] = slot;
-  if (skip) return;
-  const float4 n4 = d.m_normal[cur][slot], t04 = d.m_t0[cur][slot], t14 = d.m_t1[cur][slot];
-  d.pgs_frame[3 * k] = n4;
-  d.pgs_frame[3 * k + 1] = t04;
-  d.pgs_frame[3 * k + 2] = t14;
-  const Sym3 IA = load_iw(d, b.x), IB = load_iw(d, b.y);
-  const float3 n = f3(n4), t0 = f3(t04), t1 = f3(t14);
-  const float3 aa = f3(d.m_anchor_a[cur][slot]), ab = f3(d.m_anchor_b[cur][slot]);
-  const SoftCoef s = pgs_soft_coef(ima, imb, h, hertz);
-  for (uint32_t j = 0; j < cc; ++j) {
-    const uint32_t ci = slot * BB_MAX_CONTACTS + j;
-    float4 R1, R2, K;
-    pgs_contact_rows(d.c_pos[cur][ci], aa, ab, n, t0, t1, ima, imb, IA, IB, s, R1, R2, K);
-    d.c_r1[c0 + j] = R1;
-    d.c_r2[c0 + j] = R2;
-    d.c_k[c0 + j] = K;
-    const float4 lam = d.c_lam[cur][ci];
-    // the reference writes its mass coefficient / tangent masses into the persistent contact
-    d.pgs_lam[c0 + j] = make_float4(lam.x, lam.y, lam.z, s.mcoef);
-    const float4 kt4 = d.c_kt[cur][ci];
-    d.c_kt[cur][ci] = make_float4(R2.w, K.x, kt4.z, kt4.w);
-  }
-}
-
-// an item's two bodies: velocities and world inverse inertias
-struct PgsBodies {
-  float4 va, wa, ia0, ia1, vb, wb, ib0, ib1;
-};
-__device__ __forceinline__ PgsBodies pgs_bodies_load(const DevState& d, uint32_t a, uint32_t b) {
-  PgsBodies B;
-  B.va = d.vel[a];
-  B.wa = d.omega[a];
-  B.ia0 = d.iw[2 * a];
-  B.ia1 = d.iw[2 * a + 1];
-  B.vb = d.vel[b];
-  B.wb = d.omega[b];
-  B.ib0 = d.iw[2 * b];
-  B.ib1 = d.iw[2 * b + 1];
-  return B;
-}
-
-// mode 0: warm start, 1: solve sweep (soft bias), 2: relax sweep; B holds the item's bodies
-template <int PF, bool STAGED = true>
-__device__ __forceinline__ void pgs_item_compute(const DevState& d, const Params& p, PgsItem<PF>& x,
-                                                 const PgsBodies& B, int mode) {
-  if (x.rec.w & BB_PGS_SKIP) return;
-  const bool accum = p.flags & BB_SIM_ACCUM_IMPULSE, fric = p.flags & BB_SIM_FRICTION;
-  if (mode == 0 && !accum) return;
-  const uint32_t a = x.rec.y, b = x.rec.z, c0 = x.rec.x, cc = x.rec.w & 0xFFu;
-  const float4 va4 = B.va, vb4 = B.vb;
-  float3 va = f3(va4), wa = f3(B.wa), vb = f3(vb4), wb = f3(B.wb);
-  const Sym3 IA{B.ia0.x, B.ia0.y, B.ia0.z, B.ia0.w, B.ia1.x, B.ia1.y};
-  const Sym3 IB{B.ib0.x, B.ib0.y, B.ib0.z, B.ib0.w, B.ib1.x, B.ib1.y};
-  const float ima = x.mass.x, imb = x.mass.y, mu = x.mass.z;
-  const float3 n = f3(x.n), t0 = f3(x.t0), t1 = f3(x.t1);
-#pragma unroll
-  for (int j = 0; j < PF; ++j) {
-    if (uint32_t(j) < cc) {
-      if (mode == 0) {
-        pgs_contact_warm(f3(x.R1[j]), f3(x.R2[j]), x.lam[j], n, t0, t1, fric, ima, imb, IA, IB, va, wa, vb, wb);
-      } else {
-        pgs_contact_solve(x.R1[j], x.R2[j], x.K[j], x.lam[j], n, t0, t1, mu, mode == 1, accum, fric, ima, imb, IA,
-                          IB, va, wa, vb, wb);
-        d.pgs_lam[c0 + j] = x.lam[j];
-      }
-    }
-  }
-  if (cc > uint32_t(PF)) {  // contacts beyond the register-held ones
-    const float4* slot = pgs_extra_slot();
-    if (STAGED) cp_async_wait_all();
-    for (uint32_t j = PF; j < cc; ++j) {
-      const uint32_t ci = c0 + j;
-      const float4* e = slot + (j - PF) * 4;
-      const float4 R1 = STAGED ? e[0] : d.c_r1[ci], R2 = STAGED ? e[1] : d.c_r2[ci];
-      float4 lam = STAGED ? e[3] : d.pgs_lam[ci];
-      if (mode == 0) {
-        pgs_contact_warm(f3(R1), f3(R2), lam, n, t0, t1, fric, ima, imb, IA, IB, va, wa, vb, wb);
-      } else {
-        const float4 K = STAGED ? e[2] : d.c_k[ci];
-        pgs_contact_solve(R1, R2, K, lam, n, t0, t1, mu, mode == 1, accum, fric, ima, imb, IA, IB, va, wa, vb, wb);
-        d.pgs_lam[ci] = lam;
-      }
-    }
-  }
-  if (x.rec.w & (1u << 8)) {
-    d.vel[a] = f4(va, va4.w);
-    d.omega[a] = f4(wa, 0.f);
-  }
-  if (x.rec.w & (1u << 9)) {
-    d.vel[b] = f4(vb, vb4.w);
-    d.omega[b] = f4(wb, 0.f);
-  }
-}
-
-template <int PF, bool STAGED = true>
-__device__ __forceinline__ void pgs_item_run(const DevState& d, const Params& p, int cur, PgsItem<PF>& x, int mode) {
-  (void)cur;
-  if (x.rec.w & BB_PGS_SKIP) return;
-  if (mode == 0 && !(p.flags & BB_SIM_ACCUM_IMPULSE)) return;
-  const PgsBodies B = pgs_bodies_load(d, x.rec.y, x.rec.z);
-  pgs_item_compute<PF, STAGED>(d, p, x, B, mode);
-}
-
-// cp.async of the next item k (record r) of this thread's colour into its staging slot: the
-// bodies cannot change before this thread runs the item (the colour's items share no body),
-// and the rows and impulses are only written by the item itself.
-template <int PF>
-__device__ __forceinline__ void pgs_stage_next(const DevState& d, uint32_t k, uint4 r) {
-  float4* nb = pgs_next_base();
-  const uint32_t T = BB_PGS_THREADS, c0 = r.x, cc = min(r.w & 0xFFu, uint32_t(PF)), a = r.y, b = r.z;
-  cp_async16(nb + 0 * T, d.pgs_mass + k);
-  cp_async16(nb + 1 * T, d.pgs_frame + 3 * k);
-  cp_async16(nb + 2 * T, d.pgs_frame + 3 * k + 1);
-  cp_async16(nb + 3 * T, d.pgs_frame + 3 * k + 2);
-  for (uint32_t j = 0; j < cc; ++j) {
-    cp_async16(nb + (4 + 4 * j) * T, d.c_r1 + c0 + j);
-    cp_async16(nb + (5 + 4 * j) * T, d.c_r2 + c0 + j);
-    cp_async16(nb + (6 + 4 * j) * T, d.c_k + c0 + j);
-    cp_async16(nb + (7 + 4 * j) * T, d.pgs_lam + c0 + j);
-  }
-  cp_async16(nb + 20 * T, d.vel + a);
-  cp_async16(nb + 21 * T, d.omega + a);
-  cp_async16(nb + 22 * T, d.iw + 2 * a);
-  cp_async16(nb + 23 * T, d.iw + 2 * a + 1);
-  cp_async16(nb + 24 * T, d.vel + b);
-  cp_async16(nb + 25 * T, d.omega + b);
-  cp_async16(nb + 26 * T, d.iw + 2 * b);
-  cp_async16(nb + 27 * T, d.iw + 2 * b + 1);
-  cp_async_commit();
-}
-
-// the staged item into registers (after cp.async.wait_all); its contacts beyond PF are staged
-// in the extra slot as pgs_item_fill does
-template <int PF>
-__device__ __forceinline__ void pgs_take_next(const DevState& d, uint4 r, PgsItem<PF>& x, PgsBodies& B) {
-  const float4* nb = pgs_next_base();
-  const uint32_t T = BB_PGS_THREADS, cc = r.w & 0xFFu;
-  x.rec = r;
-  x.mass = nb[0];
-  x.n = nb[T];
-  x.t0 = nb[2 * T];
-  x.t1 = nb[3 * T];
-#pragma unroll
-  for (int j = 0; j < PF; ++j) {
-    if (uint32_t(j) < cc) {
-      x.R1[j] = nb[(4 + 4 * j) * T];
-      x.R2[j] = nb[(5 + 4 * j) * T];
-      x.K[j] = nb[(6 + 4 * j) * T];
-      x.lam[j] = nb[(7 + 4 * j) * T];
-    }
-  }
-  B.va = nb[20 * T];
-  B.wa = nb[21 * T];
-  B.ia0 = nb[22 * T];
-  B.ia1 = nb[23 * T];
-  B.vb = nb[24 * T];
-  B.wb = nb[25 * T];
-  B.ib0 = nb[26 * T];
-  B.ib1 = nb[27 * T];
-  if (cc > uint32_t(PF)) {
-    float4* slot = pgs_extra_slot();
-    for (uint32_t j = PF; j < cc; ++j) {
-      float4* e = slot + (j - PF) * 4;
-      cp_async16(e + 0, d.c_r1 + r.x + j);
-      cp_async16(e + 1, d.c_r2 + r.x + j);
-      cp_async16(e + 2, d.c_k + r.x + j);
-      cp_async16(e + 3, d.pgs_lam + r.x + j);
-    }
-    cp_async_commit();
-  }
-}
-
-// one sweep over colours 0..C-1 and the overflow bucket.  On entry x holds this thread's first
-// item of colour 0 and rec_next the record of its first item of colour 1 (or of colour 0 when
-// C == 1); on exit both are set the same way for the next sweep.  Records run one colour ahead
-// of the rest of the item, so the loads issued between barrier arrival and wait never wait on
-// an address; and they are issued after this block's arrival, so the arrival's fence does not
-// wait for them either.
-__device__ __forceinline__ uint32_t pgs_next_colour(uint32_t c, uint32_t C) { return c + 1 < C ? c + 1 : 0u; }
-
-template <int PF, bool STAGE_NEXT>
-__device__ void pgs_sweep(const DevState& d, const Params& p, int cur, int mode, const uint32_t* bs, const uint32_t* aw,
-                          uint32_t C, PgsItem<PF>& x, uint4& rec_next, uint32_t& epoch) {
-  const uint32_t tid = blockIdx.x * blockDim.x + threadIdx.x, stride = gridDim.x * blockDim.x;
-  uint32_t* sync = &d.ctr->sync_count[1];
-  for (uint32_t c = 0; c < C; ++c) {
-    // A colour whose manifolds all sleep has no work (every item is skipped) and needs no
-    // barrier: its neighbours are ordered by the barriers of the colours that do run.
-    const bool run = aw[c] != 0;
-    if (run && !STAGE_NEXT) {  // later items of the colour load after the one before has run
-      const uint32_t end = bs[c + 1];
-      for (uint32_t k = bs[c] + tid; k < end;) {
-        pgs_item_run(d, p, cur, x, mode);
-        k += stride;
-        if (k < end) pgs_item_load(d, k, x);
-      }
-    } else if (run) {
-      // The colour's first item is in x.  Its bodies and the next item's record load now; each
-      // later item (with its bodies) is staged by cp.async while the one before computes, and
-      // the record after it loads meanwhile, so a later item costs no dependent round trip.
-      const uint32_t end = bs[c + 1];
-      uint32_t k = bs[c] + tid;
-      if (k < end) {
-        uint4 rn = make_uint4(0, 0, 0, 0);
-        if (k + stride < end) rn = d.pgs_rec[k + stride];
-        PgsBodies B = pgs_bodies_load(d, x.rec.y, x.rec.z);
-        for (;;) {
-          const uint32_t kn = k + stride;
-          const bool more = kn < end;
-          uint4 rnn = make_uint4(0, 0, 0, 0);
-          if (more) {
-            pgs_stage_next<PF>(d, kn, rn);
-            if (kn + stride < end) rnn = d.pgs_rec[kn + stride];
-          }
-          pgs_item_compute<PF>(d, p, x, B, mode);
-          if (!more) break;
-          cp_async_wait_all();
-          pgs_take_next<PF>(d, rn, x, B);
-          rn = rnn;
-          k = kn;
-        }
-      }
-    }
-    const uint32_t cn = pgs_next_colour(c, C), cnn = pgs_next_colour(cn, C);
-    const uint32_t kn = bs[cn] + tid, knn = bs[cnn] + tid;
-    if (!run) {  // keep the prefetch one colour ahead
-      if (kn < bs[cn + 1]) pgs_item_load_rest(d, kn, rec_next, x);
-      if (knn < bs[cnn + 1]) rec_next = d.pgs_rec[knn];
-      continue;
-    }
-    // This colour and the next one that runs, both fitting in block 0 (items map to threads by
-    // their index in the colour), need only a CTA barrier between them: every item and every
-    // body write of both lives in block 0.  The test reads shared bucket starts and flags, so
-    // every block decides alike.
-    uint32_t ne = c + 1;
-    while (ne < C && !aw[ne]) ++ne;
-    const bool local = ne < C && bs[c + 1] - bs[c] <= blockDim.x && bs[ne + 1] - bs[ne] <= blockDim.x;
-    if (!local) grid_arrive(sync, epoch);
-    if (kn < bs[cn + 1]) pgs_item_load_rest(d, kn, rec_next, x);
-    if (knn < bs[cnn + 1]) rec_next = d.pgs_rec[knn];
-    if (local) __syncthreads();
-    else grid_wait(d.ctr, sync, epoch);
-  }
-  const uint32_t o0 = bs[BB_MAX_COLORS], o1 = bs[BB_MAX_COLORS + 1];
-  if (o0 != o1) {  // overflow bucket: serial, in manifold order
-    if (tid == 0) {
-      for (uint32_t k = o0; k < o1; ++k) {
-        PgsItem<PF> y;
-        pgs_item_load<PF, false>(d, k, y);
-        pgs_item_run<PF, false>(d, p, cur, y, mode);
-      }
-    }
-    grid_sync(d.ctr, sync, epoch);
-  }
-}
-
-// PF = 4 contacts held per item (one 255-register block per SM).  Holding fewer would let
-// two blocks share an SM but puts the other contacts' loads on the critical path, one round
-// trip each.  A streaming variant that held nothing across barriers (each item's contacts
-// copied to shared memory by cp.async while its bodies load) ran 2 or 3 blocks per SM and
-// measured slower on the 1M-box pyramids (solve 3.32 and 6.55 against 3.23 ms per substep).
-template <int PF, bool STAGE_NEXT>
-__global__ void __launch_bounds__(BB_PGS_THREADS, PF == 4 ? 1 : 2) k_pgs_soft(const DevState d, Params p, int cur, uint32_t n, float h) {
-  __shared__ uint32_t bs[BB_MAX_COLORS + 2];
-  __shared__ uint32_t aw[BB_MAX_COLORS + 1];
-  // test switch (bb_debug_wait_limit): the last block leaves, so the others' first grid barrier
-  // waits for a block that never arrives until its bounded wait gives up
-  if (gridDim.x > 1 && blockIdx.x == gridDim.x - 1 && d.ctr->abandon_block) return;
-  if (threadIdx.x < BB_MAX_COLORS + 2) bs[threadIdx.x] = d.bucket_start[threadIdx.x];
-  if (threadIdx.x < BB_MAX_COLORS + 1) aw[threadIdx.x] = d.colour_awake[threadIdx.x];
-  const uint32_t tid = blockIdx.x * blockDim.x + threadIdx.x, stride = gridDim.x * blockDim.x;
-  const bool tq = p.quirks & BB_QUIRK_INERTIA_TRANSPOSE;
-  uint32_t* sync = &d.ctr->sync_count[1];
-  uint32_t epoch = 0;
-  // the world inverse inertias and the items' records and rows were written by k_pgs_inertia
-  // and k_pgs_build before this launch
-  __syncthreads();  // bs and aw
-  const uint32_t C = d.ctr->gc_colors;
-  PgsItem<PF> x;
-  uint4 rec_next = make_uint4(0, 0, 0, 0);
-  if (C > 0 && bs[0] + tid < bs[1]) pgs_item_load(d, bs[0] + tid, x);
-  if (C > 0) {
-    const uint32_t c1 = pgs_next_colour(0, C);
-    if (bs[c1] + tid < bs[c1 + 1]) rec_next = d.pgs_rec[bs[c1] + tid];
-  }
-  pgs_sweep<PF, STAGE_NEXT>(d, p, cur, 0, bs, aw, C, x, rec_next, epoch);
-  for (uint32_t it = 0; it < p.iterations; ++it) pgs_sweep<PF, STAGE_NEXT>(d, p, cur, 1, bs, aw, C, x, rec_next, epoch);
-  if (p.flags & BB_SIM_ADVECTION) {
-    for (uint32_t i = tid; i < n; i += stride)
-      if (awake(d.flags[i])) pgs_integrate(d, i, h, tq);
-    grid_sync(d.ctr, sync, epoch);
-  }
-  for (uint32_t it = 0; it < p.relax_iterations; ++it) pgs_sweep<PF, STAGE_NEXT>(d, p, cur, 2, bs, aw, C, x, rec_next, epoch);
-  // k_pgs_writeback copies the impulses back to the persistent contacts after this launch
-}
-
-// Before k_pgs_soft, at full occupancy (the persistent kernel runs one 256-thread block per
-// SM, where these passes of one item or body per thread were latency-bound): the world
-// inverse inertias, then the records and rows of every swept item (colours and the overflow
-// bucket, [0, bucket_start[33])).  After it, the impulses back to the persistent contacts.
-__global__ void k_pgs_inertia(const DevState d, uint32_t n, Params p) {
-  const bool tq = p.quirks & BB_QUIRK_INERTIA_TRANSPOSE;
-  for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) pgs_world_inertia(d, i, tq);
-}
+// records, frames and contact rows of every swept item (the pre-step's row half; no body is
+// touched), a warp per tile
 __global__ void k_pgs_build(const DevState d, Params p, int cur, float h) {
+  __shared__ PgsTiles ft;
+  pgs_tiles(d, ft);
   const float inv_h = h > 0.f ? 1.0f / h : 0.f;
   const float hertz = fminf(p.contact_hertz, inv_h * 0.3333333333333333f);
-  const uint32_t end = d.bucket_start[BB_MAX_COLORS + 1];
+  const uint32_t T = ft.first[BB_MAX_COLORS], over = ft.start[BB_MAX_COLORS], end = ft.start[BB_MAX_COLORS + 1];
+  const uint32_t TO = T + (end - over + 31u) / 32u;  // and the overflow bucket's tiles
+  const uint32_t lane = threadIdx.x & 31u, lt = (1u << lane) - 1u, nw = gridDim.x * (blockDim.x >> 5);
   const uint32_t* list = d.bucket_vals[1];
-  for (uint32_t k = blockIdx.x * blockDim.x + threadIdx.x; k < end; k += gridDim.x * blockDim.x)
-    pgs_item_build(d, cur, k, list[k], h, hertz);
-}
-__global__ void k_pgs_writeback(const DevState d, int cur) {
-  const uint32_t M = d.ctr->manifold_count;
-  for (uint32_t k = blockIdx.x * blockDim.x + threadIdx.x; k < M; k += gridDim.x * blockDim.x) {
-    const uint32_t cc = d.pgs_cnt[k];
-    if (cc == 0) continue;
-    const uint32_t slot = d.pgs_slot[k], c0 = d.pgs_coff[k];
-    for (uint32_t j = 0; j < cc; ++j) d.c_lam[cur][slot * BB_MAX_CONTACTS + j] = d.pgs_lam[c0 + j];
-  }
-}
-
-
-
-// ---------------------------------------------------------------------------------------
-// PGS_SOFT, dataflow schedule.
-//
-// The per-colour sweeps give every body b the ordered sequence L_b of the manifolds touching
-// it, sorted by (colour, manifold) with the overflow bucket last; one sweep processes L_b in
-// that order, and a manifold's result depends only on its two bodies' states.  So instead of a
-// grid barrier after each colour, each dynamic body carries a sequence counter: item k of sweep
-// s waits until counter[b] == s * deg(b) + rank_b(k) for both its dynamic bodies, runs, and
-// releases +1 on each.  The outcome is bit-identical to the barrier schedule.
-//
-// The kernel is cooperative (all blocks resident) and thread t owns the items k = t, t + T, ...
-// of the colour-ordered list, which it runs in increasing (sweep, k) order.  Every wait points
-// at an item earlier in that order, owned by a thread that reaches it without waiting on a
-// later item of t, so the schedule cannot deadlock.  The items are the barrier schedule's
-// compact records (built by their owners), so a thread loads its next item while waiting.
-__device__ __forceinline__ void red_release_add(uint32_t* p, uint32_t v) {
-  asm volatile("red.release.gpu.global.add.u32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
-}
-__device__ __forceinline__ void flow_wait(DevCounters* c, const uint32_t* ctr, uint32_t target) {
-  uint32_t spins = 0;
-  while (ld_acquire_gpu(ctr) < target)
-    if (spin_gave_up(c, ++spins, BB_SITE_FLOW)) return;
-}
-
-// per colour-ordered item k: (rank_a | rank_b << 16, deg_a | deg_b << 16) where rank_x is the
-// item's position in L_x (colour-major, then manifold order) and deg_x = |L_x|
-__global__ void k_flow_prep(const DevState d, int cur) {
-  const uint32_t M = d.ctr->manifold_count;
-  const uint32_t* list = d.bucket_vals[1];
-  for (uint32_t k = blockIdx.x * blockDim.x + threadIdx.x; k < M; k += gridDim.x * blockDim.x) {
-    const uint32_t m = list[k];
-    const uint2 b = d.m_bodies[cur][d.man_slot[cur][m]];
-    const uint32_t cm = min(d.gc_color[m], uint32_t(BB_MAX_COLORS));
-    uint32_t rank[2] = {0, 0}, deg[2] = {0, 0};
-#pragma unroll
-    for (int q = 0; q < 2; ++q) {
-      const uint32_t x = q == 0 ? b.x : b.y;
-      if (!(d.flags[x] & BB_BODY_DYNAMIC)) continue;
-      const uint32_t s0 = d.csr_start[cur][x], s1 = d.csr_start[cur][x + 1];
-      uint32_t r = 0;
-      for (uint32_t e = s0; e < s1; ++e) {
-        const uint32_t m2 = d.csr_list[cur][e];
-        const uint32_t c2 = min(d.gc_color[m2], uint32_t(BB_MAX_COLORS));
-        r += (c2 < cm || (c2 == cm && m2 < m)) ? 1u : 0u;
-      }
-      rank[q] = r;
-      deg[q] = s1 - s0;
+  const size_t P = d.pair_capacity;
+  for (uint32_t t = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); t < TO; t += nw) {
+    uint32_t k = BB_NONE;
+    if (t < T) k = pgs_tile_item(ft, t);
+    else if (over + (t - T) * 32u + lane < end) k = over + (t - T) * 32u + lane;
+    const bool ov = t >= T;
+    const uint32_t cc = k != BB_NONE ? d.pgs_cnt[k] : 0u, c0 = k != BB_NONE ? d.pgs_coff[k] : 0u;
+    const uint32_t base = __shfl_sync(0xFFFFFFFFu, c0, 0);
+    uint32_t slot = 0;
+    float3 n{}, t0{}, t1{}, aa{}, ab{};
+    float ima = 0.f, imb = 0.f;
+    Sym3 IA{}, IB{};
+    if (k != BB_NONE) {
+      slot = d.pgs_slot[k];
+      const uint2 b = d.m_bodies[cur][slot];
+      const bool da = d.flags[b.x] & BB_BODY_DYNAMIC, db = d.flags[b.y] & BB_BODY_DYNAMIC;
+      ima = d.pos[b.x].w;
+      imb = d.pos[b.y].w;
+      n = f3(d.m_normal[cur][slot]);
+      t0 = f3(d.m_t0[cur][slot]);
+      t1 = f3(d.m_t1[cur][slot]);
+      aa = f3(d.m_anchor_a[cur][slot]);
+      ab = f3(d.m_anchor_b[cur][slot]);
+      IA = load_iw(d, b.x);
+      IB = load_iw(d, b.y);
+      const uint32_t below = ov ? 0u : (1u << d.gc_color[list[k]]) - 1u;
+      const uint32_t ma = da ? d.flow_counter[b.x] : 0u, mb = db ? d.flow_counter[b.y] : 0u;
+      d.pgs_rec[k] = make_uint4(b.x | (da ? 0x80000000u : 0u), b.y | (db ? 0x80000000u : 0u),
+                                cc | uint32_t(__popc(ma & below)) << 4 | uint32_t(__popc(ma)) << 9 |
+                                    uint32_t(__popc(mb & below)) << 15 | uint32_t(__popc(mb)) << 20,
+                                ov ? c0 : base);
+      d.pgs_frame[k] = f4(n, ima);
+      d.pgs_frame[P + k] = f4(t0, imb);
+      d.pgs_frame[2 * P + k] = f4(t1, sqrtf(d.iinv[b.x].w * d.iinv[b.y].w));
+      d.pgs_mass[k] = f4(aa, ab.x);
+      pgs_anchor(d)[k] = make_float2(ab.y, ab.z);
     }
-    d.flow_rec[k] = make_uint4((rank[0] & 0xFFFFu) | (rank[1] << 16), (deg[0] & 0xFFFFu) | (deg[1] << 16), 0u, 0u);
+    const SoftCoef s = pgs_soft_coef(ima, imb, h, hertz);
+    uint32_t off = base;
+    for (uint32_t j = 0;; ++j) {
+      const uint32_t m = __ballot_sync(0xFFFFFFFFu, cc > j);
+      if (m == 0u) break;
+      if (cc > j) {
+        const size_t ci = size_t(slot) * BB_MAX_CONTACTS + j, r = ov ? c0 + j : off + uint32_t(__popc(m & lt));
+        const float4 pp = d.c_pos[cur][ci];
+        float4 R1, R2, K;
+        pgs_contact_rows(pp, aa, ab, n, t0, t1, ima, imb, IA, IB, s, R1, R2, K);
+        const float4 lam = d.c_lam[cur][ci];
+        d.c_r1[r] = f4(f3(pp), R1.w);
+        pgs_tmass(d)[r] = make_float2(R2.w, K.x);
+        d.pgs_lam[r] = make_float4(lam.x, lam.y, lam.z, K.y);
+        // the reference writes its tangent masses into the persistent contact
+        const float4 kt4 = d.c_kt[cur][ci];
+        d.c_kt[cur][ci] = make_float4(R2.w, K.x, kt4.z, kt4.w);
+      }
+      off += uint32_t(__popc(m));
+    }
   }
 }
 
-// world inverse inertia cache and zeroed sequence counters
-__global__ void k_flow_init(const DevState d, Params p, uint32_t n) {
-  uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  pgs_world_inertia(d, i, p.quirks & BB_QUIRK_INERTIA_TRANSPOSE);
-  d.flow_counter[i] = 0;
-}
-
-// one dataflow sweep s (mode 0 warm start, 1 solve, 2 relax) over this thread's items
-template <int PF>
-__device__ void flow_sweep(const DevState& d, const Params& p, int cur, uint32_t s, int mode, uint32_t M, PgsItem<PF>& x,
-                           uint4& fr) {
-  const uint32_t tid = blockIdx.x * blockDim.x + threadIdx.x, stride = gridDim.x * blockDim.x;
-  for (uint32_t k = tid; k < M; k += stride) {
-    const uint32_t a = x.rec.y, b = x.rec.z;
-    const bool da = x.rec.w & (1u << 8), db = x.rec.w & (1u << 9);
-    if (da) flow_wait(d.ctr, &d.flow_counter[a], s * (fr.y & 0xFFFFu) + (fr.x & 0xFFFFu));
-    if (db) flow_wait(d.ctr, &d.flow_counter[b], s * (fr.y >> 16) + (fr.x >> 16));
-    pgs_item_run(d, p, cur, x, mode);
-    if (da) red_release_add(&d.flow_counter[a], 1u);
-    if (db) red_release_add(&d.flow_counter[b], 1u);
-    // this thread's next item (wrapping to its first for the next sweep)
-    const uint32_t kn = k + stride < M ? k + stride : tid;
-    pgs_item_load(d, kn, x);
-    fr = d.flow_rec[kn];
+// contacts [first, first + BB_PGS_PF) of a tile's lanes, and where their impulses live
+struct PgsRows {
+  float4 A[BB_PGS_PF], L[BB_PGS_PF];
+  float2 B[BB_PGS_PF];
+  uint32_t at[BB_PGS_PF];
+};
+__device__ __forceinline__ void pgs_rows_load(const DevState& d, uint32_t cc, uint32_t first, uint32_t& off, PgsRows& x) {
+  const uint32_t lt = (1u << (threadIdx.x & 31u)) - 1u;
+#pragma unroll
+  for (int j = 0; j < BB_PGS_PF; ++j) {
+    const bool has = cc > first + uint32_t(j);
+    const uint32_t m = __ballot_sync(0xFFFFFFFFu, has);
+    x.at[j] = off + uint32_t(__popc(m & lt));
+    off += uint32_t(__popc(m));
+    if (has) {
+      x.A[j] = d.c_r1[x.at[j]];
+      x.B[j] = pgs_tmass(d)[x.at[j]];
+      x.L[j] = d.pgs_lam[x.at[j]];
+    }
   }
 }
 
-template <int PF>
-__global__ void __launch_bounds__(BB_PGS_THREADS, PF == 4 ? 1 : 2) k_pgs_flow(const DevState d, Params p, int cur,
-                                                                               uint32_t n, float h) {
+struct PgsItem {
+  float3 n, t0, t1, aa, ab;
+  float ima, imb, mu;
+};
+__device__ __forceinline__ PgsItem pgs_item_load(const DevState& d, uint32_t k) {
+  const size_t P = d.pair_capacity;
+  const float4 f0 = d.pgs_frame[k], f1 = d.pgs_frame[P + k], f2 = d.pgs_frame[2 * P + k], f3_ = d.pgs_mass[k];
+  const float2 g = pgs_anchor(d)[k];
+  PgsItem x;
+  x.n = f3(f0);
+  x.ima = f0.w;
+  x.t0 = f3(f1);
+  x.imb = f1.w;
+  x.t1 = f3(f2);
+  x.mu = f2.w;
+  x.aa = f3(f3_);
+  x.ab = make_float3(f3_.w, g.x, g.y);
+  return x;
+}
+
+// the two soft-coefficient pairs (solvers.slang:150-158): a contact with a static body, and not
+struct PgsCoef {
+  float m[2], i[2];
+};
+
+// one contact of an item: warm start (mode 0), solve sweep (1) or relax sweep (2)
+__device__ __forceinline__ void pgs_run_contact(const PgsItem& x, float4 A, float2 B, float4& L, int mode, bool accum,
+                                                bool fric, const PgsCoef& co, const Sym3& IA, const Sym3& IB, float3& va,
+                                                float3& wa, float3& vb, float3& wb) {
+  const float3 r1 = xsub(f3(A), x.aa), r2 = xsub(f3(A), x.ab);
+  if (mode == 0) {
+    pgs_contact_warm(r1, r2, L, x.n, x.t0, x.t1, fric, x.ima, x.imb, IA, IB, va, wa, vb, wb);
+  } else {
+    const int q = (x.ima == 0.f || x.imb == 0.f) ? 1 : 0;
+    const float bias = L.w;
+    float4 lam = L;
+    pgs_contact_solve(f4(r1, A.w), f4(r2, B.x), make_float4(B.y, bias, q ? co.m[1] : co.m[0], q ? co.i[1] : co.i[0]), lam,
+                      x.n, x.t0, x.t1, x.mu, mode == 1, accum, fric, x.ima, x.imb, IA, IB, va, wa, vb, wb);
+    L = make_float4(lam.x, lam.y, lam.z, bias);
+  }
+}
+
+// gives up a tagged wait past the world's limit, or when another wait already did
+__device__ __forceinline__ bool pgs_gave_up(DevCounters* c, uint32_t spins) {
+  if ((spins & 63u) != 0u) return false;
+  const uint32_t lim = *reinterpret_cast<volatile const uint32_t*>(&c->wait_limit);
+  if (spins > (lim ? lim : BB_SPIN_LIMIT)) {
+    raise_wait_error(c, BB_SITE_FLOW);
+    return true;
+  }
+  return (*reinterpret_cast<volatile const uint32_t*>(&c->error_flags) & BB_ERRF_SPIN_LIMIT) != 0;
+}
+
+// sweeps [s0, s1): those below warm are the warm start, those below mid solve, the rest relax
+__device__ __forceinline__ void pgs_sweeps(const DevState& d, const Params& p, const PgsTiles& ft, const PgsCoef& co,
+                                           uint32_t s0, uint32_t s1, uint32_t warm, uint32_t mid, bool& dead) {
+  const uint32_t T = ft.first[BB_MAX_COLORS];
+  const uint32_t w0 = (threadIdx.x >> 5) * gridDim.x + blockIdx.x, nw = gridDim.x * (BB_PGS_THREADS / 32);
+  if (w0 >= T || s0 >= s1) return;
+  const bool accum = p.flags & BB_SIM_ACCUM_IMPULSE, fric = p.flags & BB_SIM_FRICTION;
+  const bool single = w0 + nw >= T;  // this warp's only tile stays in registers
+  float4* vw = pgs_vw(d);
+  uint32_t t = w0, s = s0;
+  uint32_t k = pgs_tile_item(ft, t);
+  uint4 rec = make_uint4(0, 0, 0, 0);
+  if (k != BB_NONE) rec = d.pgs_rec[k];
+  PgsItem x;
+  PgsRows r;
+  Sym3 IA, IB;
+  bool fresh = true;
+  uint32_t off = 0;
+  for (;;) {
+    // this warp's next tile and its record, a tile ahead
+    uint32_t tn = t + nw, sn = s;
+    if (tn >= T) {
+      tn = w0;
+      ++sn;
+    }
+    const uint32_t kn = pgs_tile_item(ft, tn);
+    uint4 rn = make_uint4(0, 0, 0, 0);
+    if (kn != BB_NONE) rn = d.pgs_rec[kn];
+    const bool on = k != BB_NONE;
+    const uint32_t a = PGS_BODY(rec.x), b = PGS_BODY(rec.y), cc = rec.z & 15u;
+    const uint32_t na = s * ((rec.z >> 9) & 63u) + ((rec.z >> 4) & 31u), nb = s * (rec.z >> 20) + ((rec.z >> 15) & 31u);
+    // The body loads go first: their first round trip overlaps the rows'.
+    float4 va4, wa4, vb4, wb4;
+    va4 = wa4 = vb4 = wb4 = make_float4(0.f, 0.f, 0.f, 0.f);
+    auto bodies = [&](bool la, bool lb) {
+      if (la) {
+        va4 = ld_tagged(vw + 2 * size_t(a));
+        wa4 = ld_tagged(vw + 2 * size_t(a) + 1);
+      }
+      if (lb) {
+        vb4 = ld_tagged(vw + 2 * size_t(b));
+        wb4 = ld_tagged(vw + 2 * size_t(b) + 1);
+      }
+    };
+    bodies(on, on);
+    if (fresh) {
+      off = __shfl_sync(0xFFFFFFFFu, rec.w, 0);
+      if (on) {
+        x = pgs_item_load(d, k);
+        IA = load_iw(d, a);
+        IB = load_iw(d, b);
+      }
+      pgs_rows_load(d, cc, 0, off, r);
+    }
+    // the rows beyond the first BB_PGS_PF contacts, for tiles that have them
+    const bool deep = __any_sync(0xFFFFFFFFu, cc > BB_PGS_PF);
+    PgsRows y;
+    if (deep) {
+      uint32_t off2 = off;
+      pgs_rows_load(d, cc, BB_PGS_PF, off2, y);
+    }
+    for (uint32_t spins = 0;;) {
+      const bool okA = !on || (__float_as_uint(va4.w) == na && __float_as_uint(wa4.w) == na);
+      const bool okB = !on || (__float_as_uint(vb4.w) == nb && __float_as_uint(wb4.w) == nb);
+      if (__all_sync(0xFFFFFFFFu, okA && okB) || dead) break;
+      bodies(!okA, !okB);
+      dead = __any_sync(0xFFFFFFFFu, pgs_gave_up(d.ctr, ++spins));
+    }
+    const int mode = s < warm ? 0 : s < mid ? 1 : 2;
+    float3 va = f3(va4), wa = f3(wa4), vb = f3(vb4), wb = f3(wb4);
+#pragma unroll
+    for (int j = 0; j < BB_PGS_PF; ++j)
+      if (cc > uint32_t(j)) pgs_run_contact(x, r.A[j], r.B[j], r.L[j], mode, accum, fric, co, IA, IB, va, wa, vb, wb);
+    if (deep) {
+#pragma unroll
+      for (int j = 0; j < BB_PGS_PF; ++j)
+        if (cc > uint32_t(BB_PGS_PF + j))
+          pgs_run_contact(x, y.A[j], y.B[j], y.L[j], mode, accum, fric, co, IA, IB, va, wa, vb, wb);
+    }
+    // the bodies first: other warps wait for them
+    if (rec.x >> 31) {
+      st_tagged(vw + 2 * size_t(a), va, na + 1u);
+      st_tagged(vw + 2 * size_t(a) + 1, wa, na + 1u);
+    }
+    if (rec.y >> 31) {
+      st_tagged(vw + 2 * size_t(b), vb, nb + 1u);
+      st_tagged(vw + 2 * size_t(b) + 1, wb, nb + 1u);
+    }
+    if (mode != 0) {
+#pragma unroll
+      for (int j = 0; j < BB_PGS_PF; ++j) {
+        if (cc > uint32_t(j)) d.pgs_lam[r.at[j]] = r.L[j];
+        if (deep && cc > uint32_t(BB_PGS_PF + j)) d.pgs_lam[y.at[j]] = y.L[j];
+      }
+    }
+    if (sn >= s1) return;
+    t = tn;
+    s = sn;
+    k = kn;
+    rec = rn;
+    fresh = !single;
+  }
+}
+
+// an item of the overflow bucket, run serially between grid barriers: tags stay as they are
+__device__ __forceinline__ void pgs_overflow_item(const DevState& d, const Params& p, uint32_t k, int mode,
+                                                  const PgsCoef& co) {
+  const uint4 rec = d.pgs_rec[k];
+  const bool accum = p.flags & BB_SIM_ACCUM_IMPULSE, fric = p.flags & BB_SIM_FRICTION;
+  const uint32_t a = PGS_BODY(rec.x), b = PGS_BODY(rec.y), cc = rec.z & 15u;
+  const PgsItem x = pgs_item_load(d, k);
+  const Sym3 IA = load_iw(d, a), IB = load_iw(d, b);
+  float4* vw = pgs_vw(d);
+  const float4 va4 = ld_tagged(vw + 2 * size_t(a)), wa4 = ld_tagged(vw + 2 * size_t(a) + 1);
+  const float4 vb4 = ld_tagged(vw + 2 * size_t(b)), wb4 = ld_tagged(vw + 2 * size_t(b) + 1);
+  float3 va = f3(va4), wa = f3(wa4), vb = f3(vb4), wb = f3(wb4);
+  for (uint32_t j = rec.w; j < rec.w + cc; ++j) {
+    float4 L = d.pgs_lam[j];
+    pgs_run_contact(x, d.c_r1[j], pgs_tmass(d)[j], L, mode, accum, fric, co, IA, IB, va, wa, vb, wb);
+    d.pgs_lam[j] = L;
+  }
+  if (rec.x >> 31) {
+    st_tagged(vw + 2 * size_t(a), va, __float_as_uint(va4.w));
+    st_tagged(vw + 2 * size_t(a) + 1, wa, __float_as_uint(wa4.w));
+  }
+  if (rec.y >> 31) {
+    st_tagged(vw + 2 * size_t(b), vb, __float_as_uint(vb4.w));
+    st_tagged(vw + 2 * size_t(b) + 1, wb, __float_as_uint(wb4.w));
+  }
+}
+
+__global__ void __launch_bounds__(BB_PGS_THREADS, BB_PGS_PER_SM) k_pgs_soft(const DevState d, Params p, uint32_t n, float h) {
+  __shared__ PgsTiles ft;
+  // test switch (bb_debug_wait_limit): the last block leaves, so the others' waits for it run out
+  if (gridDim.x > 1 && blockIdx.x == gridDim.x - 1 && d.ctr->abandon_block) return;
+  pgs_tiles(d, ft);
   const uint32_t tid = blockIdx.x * blockDim.x + threadIdx.x, stride = gridDim.x * blockDim.x;
   const bool tq = p.quirks & BB_QUIRK_INERTIA_TRANSPOSE;
   const float inv_h = h > 0.f ? 1.0f / h : 0.f;
   const float hertz = fminf(p.contact_hertz, inv_h * 0.3333333333333333f);
+  const SoftCoef c0 = pgs_soft_coef(1.f, 1.f, h, hertz), c1 = pgs_soft_coef(0.f, 1.f, h, hertz);
+  const PgsCoef co{{c0.mcoef, c1.mcoef}, {c0.icoef, c1.icoef}};
   uint32_t* sync = &d.ctr->sync_count[1];
   uint32_t epoch = 0;
-  const uint32_t M = d.ctr->manifold_count;
-  const uint32_t* list = d.bucket_vals[1];
-  for (uint32_t k = tid; k < M; k += stride) pgs_item_build(d, cur, k, list[k], h, hertz);
-  PgsItem<PF> x;
-  uint4 fr = make_uint4(0, 0, 0, 0);
-  if (tid < M) {
-    pgs_item_load(d, tid, x);
-    fr = d.flow_rec[tid];
-  }
-  uint32_t s = 0;
-  flow_sweep(d, p, cur, s++, 0, M, x, fr);
-  for (uint32_t it = 0; it < p.iterations; ++it) flow_sweep(d, p, cur, s++, 1, M, x, fr);
-  if (p.flags & BB_SIM_ADVECTION) {
-    grid_sync(d.ctr, sync, epoch);
-    for (uint32_t i = tid; i < n; i += stride)
-      if (awake(d.flags[i])) pgs_integrate(d, i, h, tq);
-    grid_sync(d.ctr, sync, epoch);
-  }
-  for (uint32_t it = 0; it < p.relax_iterations; ++it) flow_sweep(d, p, cur, s++, 2, M, x, fr);
-  grid_sync(d.ctr, sync, epoch);
-  for (uint32_t k = tid; k < M; k += stride) {  // impulses back to the persistent contacts
-    const uint32_t cc = d.pgs_cnt[k];
-    if (cc == 0) continue;
-    const uint32_t slot = d.pgs_slot[k], c0 = d.pgs_coff[k];
-    for (uint32_t j = 0; j < cc; ++j) d.c_lam[cur][slot * BB_MAX_CONTACTS + j] = d.pgs_lam[c0 + j];
+  float4* vw = pgs_vw(d);
+  bool dead = false;
+  const uint32_t warm = (p.flags & BB_SIM_ACCUM_IMPULSE) ? 1u : 0u, mid = warm + p.iterations, last = mid + p.relax_iterations;
+  const uint32_t o0 = ft.start[BB_MAX_COLORS], o1 = ft.start[BB_MAX_COLORS + 1];
+  bool integrated = !(p.flags & BB_SIM_ADVECTION);
+  for (uint32_t s = 0;;) {
+    if (s == mid && !integrated) {
+      grid_sync(d.ctr, sync, epoch);
+      for (uint32_t i = tid; i < n; i += stride)
+        if (awake(d.flags[i]))
+          pgs_integrate_body(d.pos, d.rot, vw[2 * size_t(i)], vw[2 * size_t(i) + 1], d.iinv, d.iinv_off,
+                             d.full_inertia != 0, d.iw, i, h, tq);
+      grid_sync(d.ctr, sync, epoch);
+      integrated = true;
+    }
+    if (s >= last) break;
+    const uint32_t e = o0 != o1 ? s + 1u : s < mid ? mid : last;
+    pgs_sweeps(d, p, ft, co, s, e, warm, mid, dead);
+    if (o0 != o1) {  // overflow bucket: serial, in manifold order
+      grid_sync(d.ctr, sync, epoch);
+      if (tid == 0)
+        for (uint32_t k = o0; k < o1; ++k) pgs_overflow_item(d, p, k, s < warm ? 0 : s < mid ? 1 : 2, co);
+      grid_sync(d.ctr, sync, epoch);
+    }
+    s = e;
   }
 }
 
-int bb_pgs_soft_blocks(int sms) {
-  cudaFuncSetAttribute((const void*)k_pgs_soft<4, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, BB_PGS_SMEM_EXTRA);
-  cudaFuncSetAttribute((const void*)k_pgs_soft<4, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, BB_PGS_SMEM);
-  cudaFuncSetAttribute((const void*)k_pgs_flow<4>, cudaFuncAttributeMaxDynamicSharedMemorySize, BB_PGS_SMEM_EXTRA);
-  return bb_coop_blocks((const void*)k_pgs_soft<4, false>, BB_PGS_THREADS, sms);
+// after the sweeps: impulses back to the persistent contacts (with the mass coefficient the
+// reference leaves there), velocities back to the bodies
+__global__ void k_pgs_finish(const DevState d, Params p, int cur, uint32_t n, float h) {
+  __shared__ PgsTiles ft;
+  pgs_tiles(d, ft);
+  const float inv_h = h > 0.f ? 1.0f / h : 0.f;
+  const float hertz = fminf(p.contact_hertz, inv_h * 0.3333333333333333f);
+  const uint32_t T = ft.first[BB_MAX_COLORS], over = ft.start[BB_MAX_COLORS], end = ft.start[BB_MAX_COLORS + 1];
+  const uint32_t TO = T + (end - over + 31u) / 32u;
+  const uint32_t lane = threadIdx.x & 31u, lt = (1u << lane) - 1u, nw = gridDim.x * (blockDim.x >> 5);
+  for (uint32_t t = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); t < TO; t += nw) {
+    uint32_t k = BB_NONE;
+    if (t < T) k = pgs_tile_item(ft, t);
+    else if (over + (t - T) * 32u + lane < end) k = over + (t - T) * 32u + lane;
+    const bool ov = t >= T;
+    const uint32_t cc = k != BB_NONE ? d.pgs_cnt[k] : 0u, c0 = k != BB_NONE ? d.pgs_coff[k] : 0u;
+    uint32_t off = __shfl_sync(0xFFFFFFFFu, c0, 0), slot = 0;
+    float mcoef = 0.f;
+    if (k != BB_NONE) {
+      slot = d.pgs_slot[k];
+      mcoef = pgs_soft_coef(d.pgs_frame[k].w, d.pgs_frame[size_t(d.pair_capacity) + k].w, h, hertz).mcoef;
+    }
+    for (uint32_t j = 0;; ++j) {
+      const uint32_t m = __ballot_sync(0xFFFFFFFFu, cc > j);
+      if (m == 0u) break;
+      if (cc > j) {
+        const float4 L = d.pgs_lam[ov ? c0 + j : off + uint32_t(__popc(m & lt))];
+        d.c_lam[cur][size_t(slot) * BB_MAX_CONTACTS + j] = make_float4(L.x, L.y, L.z, mcoef);
+      }
+      off += uint32_t(__popc(m));
+    }
+  }
+  const float4* vw = pgs_vw(d);
+  for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+    if (!(d.flags[i] & BB_BODY_DYNAMIC)) continue;
+    d.vel[i] = f4(f3(vw[2 * size_t(i)]), d.vel[i].w);
+    d.omega[i] = f4(f3(vw[2 * size_t(i) + 1]), 0.f);
+  }
+}
+
+// blocks of k_pgs_soft per SM (one unit of its grid) that are resident together
+static int pgs_blocks_per_sm() {
+  int per_sm = 0;
+  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, (const void*)k_pgs_soft, BB_PGS_THREADS, 0);
+  return std::max(1, std::min(per_sm, BB_PGS_PER_SM));
+}
+
+// Grid: as many SMs' worth of blocks as 256-thread groups fit the largest colour (about half the
+// bodies), so a small world leaves the rest of the GPU to other streams.
+int bb_pgs_soft_blocks(int sms, uint32_t max_bodies) {
+  const uint64_t groups = (uint64_t(max_bodies) / 2 + 255) / 256;
+  return int(std::max<uint64_t>(1, std::min<uint64_t>(uint64_t(sms), groups))) * pgs_blocks_per_sm();
 }
 
 void bb_solve_pgs_soft(cudaStream_t s, const DevState& d, const Params& p, uint32_t n, float h, int cur,
                        const StepScratch& sc, int coop_blocks, int sms) {
-  cudaMemsetAsync(d.colour_awake, 0, sizeof(uint32_t) * (BB_MAX_COLORS + 1), s);
-  k_pgs_count<<<sms * 8, BB_THREADS, 0, s>>>(d, cur);
-  bb_launch_scan(s, d.pgs_cnt, d.pgs_coff, &d.ctr->manifold_count, d.pair_capacity, &d.ctr->pgs_contacts,
+  if (n == 0) return;
+  const int T = BB_THREADS;
+  const uint32_t blocks = (n + T - 1) / T;
+  k_pgs_bodies<<<blocks, T, 0, s>>>(d, n, p);
+  k_pgs_count<<<sms * 8, T, 0, s>>>(d, cur);
+  bb_launch_scan(s, d.pgs_cnt, d.pgs_coff, &d.bucket_start[BB_MAX_COLORS + 1], d.pair_capacity, &d.ctr->pgs_contacts,
                  sc.scan_status + 4 * size_t(sc.scan_tiles), sc.scan_tile_ctr + 4, d.ctr);
-  if (p.schedule == BB_SCHEDULE_DATAFLOW) {
-    k_flow_prep<<<sms * 8, BB_THREADS, 0, s>>>(d, cur);
-    k_flow_init<<<(n + BB_THREADS - 1) / BB_THREADS, BB_THREADS, 0, s>>>(d, p, n);
-    DevState dd = d;
-    Params pp = p;
-    int cc = cur;
-    uint32_t nn = n;
-    float hh = h;
-    void* args[] = {&dd, &pp, &cc, &nn, &hh};
-    const void* kern = (const void*)k_pgs_flow<4>;
-    bb_launch_coop(kern, coop_blocks, BB_PGS_THREADS, args, s, BB_PGS_SMEM_EXTRA);
-    return;
-  }
+  k_pgs_build<<<sms * 8, T, 0, s>>>(d, p, cur, h);
   DevState dd = d;
   Params pp = p;
-  int cc = cur;
   uint32_t nn = n;
   float hh = h;
-  void* args[] = {&dd, &pp, &cc, &nn, &hh};
-  if (n) k_pgs_inertia<<<(n + BB_THREADS - 1) / BB_THREADS, BB_THREADS, 0, s>>>(d, n, p);
-  k_pgs_build<<<sms * 8, BB_THREADS, 0, s>>>(d, p, cur, h);
-  // staging the next item needs 112 KB more shared memory (less L1): it pays when threads run
-  // several items per colour (large worlds), which is what the autotuner measures
-  if (p.pgs_stage_next)
-    bb_launch_coop((const void*)k_pgs_soft<4, true>, coop_blocks, BB_PGS_THREADS, args, s, BB_PGS_SMEM);
-  else bb_launch_coop((const void*)k_pgs_soft<4, false>, coop_blocks, BB_PGS_THREADS, args, s, BB_PGS_SMEM_EXTRA);
-  k_pgs_writeback<<<sms * 8, BB_THREADS, 0, s>>>(d, cur);
+  void* args[] = {&dd, &pp, &nn, &hh};
+  bb_launch_coop((const void*)k_pgs_soft, coop_blocks, BB_PGS_THREADS, args, s);
+  k_pgs_finish<<<sms * 8, T, 0, s>>>(d, p, cur, n, h);
 }
 
 // ---------------------------------------------------------------------------------------
@@ -1069,7 +969,7 @@ void bb_solve_islands(cudaStream_t s, const DevState& d, const Params& p, uint32
   if (n == 0) return;
   const int T = BB_THREADS;
   const uint32_t blocks = (n + T - 1) / T;
-  k_flow_init<<<blocks, T, 0, s>>>(d, p, n);  // world inverse inertia of every body
+  k_pgs_bodies<<<blocks, T, 0, s>>>(d, n, p);  // world inverse inertia of every body
   k_island_keys<<<sms * 8, T, 0, s>>>(d, cur);
   uint32_t* keys[2] = {d.bucket_keys[0], d.bucket_keys[1]};
   uint32_t* vals[2] = {d.bucket_vals[0], d.bucket_vals[1]};

@@ -765,7 +765,7 @@ bb_status bb_world_create(const bb_world_desc* desc, void** out_world) {
     return int(std::max<uint64_t>(1, std::min<uint64_t>(uint64_t(max_blocks), (items + threads - 1) / threads)));
   };
   w->coop_edge = fit(bb_edge_coloring_blocks(w->sms), w->cap_n, 1024);
-  w->coop_pgs = fit(bb_pgs_soft_blocks(w->sms), w->cap_n / 2, 256);
+  w->coop_pgs = bb_pgs_soft_blocks(w->sms, w->cap_n);
   onesweep_smem_attr();
   w->coop_avbd = fit(bb_avbd_blocks(w->sms), w->cap_n / 2, 512);
   w->coop_cc = fit(bb_components_blocks(w->sms), w->cap_n, 512);
@@ -1894,18 +1894,13 @@ bb_status bb_autotune(void* world, float dt, uint32_t substeps, uint32_t trial_s
   struct Axis {
     uint32_t bb_solver_params::*field;
     std::vector<uint32_t> values;
-    bool pgs_only, barrier_only;
   };
   const std::vector<Axis> axes = {
-      {&bb_solver_params::schedule, {BB_SCHEDULE_DATAFLOW, BB_SCHEDULE_COLOUR_BARRIER}, true, false},
-      {&bb_solver_params::broad_threads, {32, 64, 128}, false, false},
-      {&bb_solver_params::narrow_blocks_per_sm, {4, 8, 16, 32}, false, false},
-      {&bb_solver_params::pgs_stage_next, {0, 1}, true, true},
+      {&bb_solver_params::broad_threads, {32, 64, 128}},
+      {&bb_solver_params::narrow_blocks_per_sm, {4, 8, 16, 32}},
   };
   for (const Axis& ax : axes) {
     if (st != BB_OK) break;
-    if (ax.pgs_only && best.solver != BB_SOLVER_PGS_SOFT) continue;
-    if (ax.barrier_only && best.schedule != BB_SCHEDULE_COLOUR_BARRIER) continue;
     for (uint32_t v : ax.values) {
       if (best.*ax.field == v) continue;
       bb_solver_params cand = best;

@@ -94,10 +94,10 @@ typedef int32_t bb_status;
 #define BB_BOUNDS_AUTO 1u  /* per substep: min/max of body positions */
 
 /* ---- colour-sweep schedules ------------------------------------------------------------
- * DATAFLOW: every (sweep, manifold) item waits on per-body sequence counters for exactly the
- * items that precede it on its two bodies in (sweep, colour, manifold) order -- the order the
- * reference's per-colour dispatches impose -- so no grid-wide barrier is needed.
- * COLOUR_BARRIER: one grid barrier between colours, as the reference's dispatch sequence. */
+ * Both values run the same kernel: every (sweep, manifold) item waits for exactly the items that
+ * precede it on its two bodies in (sweep, colour, manifold) order, the order that the
+ * reference's per-colour dispatches impose.  (They named two kernels with the same results;
+ * the field is kept for callers that set it.) */
 #define BB_SCHEDULE_DATAFLOW 0u
 #define BB_SCHEDULE_COLOUR_BARRIER 1u
 
@@ -138,8 +138,7 @@ typedef struct bb_solver_params {
   /* launch geometry (results are identical for every value; 0 = default; bb_autotune picks) */
   uint32_t broad_threads;        /* broad-phase block size: 32, 64 or 128 (default 128) */
   uint32_t narrow_blocks_per_sm; /* narrow-phase grid, 128-thread blocks per SM: 1..64 (default 16) */
-  uint32_t pgs_stage_next;       /* colour-barrier PGS_SOFT: 1 stages each thread's next item of a colour in shared
-                                    memory while the current one computes (large worlds); 0 loads it after (default) */
+  uint32_t pgs_stage_next;       /* 0 (default) or 1; no effect (kept for callers that set it) */
   /* Morton normalisation */
   uint32_t bounds_mode;        /* BB_BOUNDS_* */
   float world_min[3];          /* default -64 */
@@ -201,7 +200,7 @@ typedef struct bb_step_stats {
   uint32_t solved_contacts;       /* and their contacts (0 under AVBD and the per-island path) */
   uint32_t graph_color_rounds;    /* bid/commit rounds the last edge colouring ran (at most gc_rounds) */
   uint32_t error_site;            /* where the first bounded wait gave up (BB_ERRF_SPIN_LIMIT): 0 none,
-                                     1 sort look-back, 2 dataflow PGS wait, 3 generation barrier, 4 scan
+                                     1 sort look-back, 2 PGS_SOFT wait for a body, 3 generation barrier, 4 scan
                                      look-back, 16 + k grid barrier k (0 edge colouring, 1 PGS_SOFT, 2 AVBD
                                      colouring, 3..5 AVBD solve phases, 7 connected components) */
 } bb_step_stats;
@@ -462,8 +461,8 @@ bb_status bb_radix_sort_pairs_static(const uint32_t* keys_in, const uint32_t* va
  * sort passes clamp silently, LBVH.slang:34-152). */
 bb_status bb_radix_sort_error_flags(uint32_t static_scratch, void* stream, uint32_t* error_flags);
 
-/* Pick the launch geometry and colour-sweep schedule of this world by timing candidates
- * (coordinate descent over bb_solver_params.schedule, broad_threads, narrow_blocks_per_sm,
+/* Pick the launch geometry of this world by timing candidates
+ * (coordinate descent over bb_solver_params.broad_threads, narrow_blocks_per_sm;
  * pgs_stage_next; each candidate timed between two runs of the incumbent).  All candidates
  * give bit-identical results, so the trial steps are ordinary steps (about 21 x
  * (trial_steps + 1) of them): use it in place of warm-up.  The
