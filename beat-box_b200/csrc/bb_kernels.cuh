@@ -55,7 +55,7 @@ void bb_solve_islands(cudaStream_t s, const DevState& d, const Params& p, uint32
 void bb_solve_pgs_soft(cudaStream_t s, const DevState& d, const Params& p, uint32_t n, float h, int cur,
                        const StepScratch& sc, int coop_blocks, int sms);
 void bb_solve_avbd(cudaStream_t s, const DevState& d, const Params& p, uint32_t n, float h, const StepScratch& sc,
-                   int sms, int cur, int coop_blocks);
+                   int sms, int cur, int coop_blocks, int color_blocks);
 
 // serving loop helpers (bb_world.cu): one batch slot's state, the device error word
 bb_status bb_world_read_range(void* world, uint32_t first, uint32_t count, float* position, float* rotation,
@@ -75,7 +75,8 @@ void bb_sort_carve(char* base, uint32_t n, int passes, DevCounters** ctr, uint32
 // co-resident block counts of the persistent cooperative kernels
 int bb_edge_coloring_blocks(int sms);
 int bb_pgs_soft_blocks(int sms, uint32_t max_bodies);
-int bb_avbd_blocks(int sms);
+int bb_avbd_blocks(int sms, uint32_t max_bodies);
+int bb_avbd_color_blocks(int sms);
 
 // occupancy helpers (bb_world.cu)
 int bb_coop_blocks(const void* kernel, int threads, int sms);

@@ -1059,6 +1059,13 @@ __global__ void __launch_bounds__(BB_COOP_THREADS, 1) k_avbd_color(const DevStat
   }
 }
 
+// displacement of body i since the step's start, linear and angular (the AVBD sweeps read a
+// partner's 32 bytes here instead of its pose and start pose)
+__device__ __forceinline__ void avbd_store_disp(const DevState& d, uint32_t i, float3 dp, float3 dth) {
+  d.iw[2 * size_t(i)] = f4(dp, 0.f);
+  d.iw[2 * size_t(i) + 1] = f4(dth, 0.f);
+}
+
 __global__ void k_avbd_prepare(const DevState d, Params p, uint32_t n, float dt) {
   uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
@@ -1085,8 +1092,10 @@ __global__ void k_avbd_prepare(const DevState d, Params p, uint32_t n, float dt)
     float sg = grav > 0.f ? 1.f : -1.f;
     aw = fminf(fmaxf(ay * sg / fabsf(grav), 0.f), 1.f);
   }
-  d.pos[i] = f4(pos + v * dt + make_float3(0.f, grav, 0.f) * (aw * dt * dt), ps.w);
+  const float3 pn = pos + v * dt + make_float3(0.f, grav, 0.f) * (aw * dt * dt);
+  d.pos[i] = f4(pn, ps.w);
   d.rot[i] = q_to4(qt);
+  avbd_store_disp(d, i, pn - pos, small_angle_delta(qt, q));
 }
 
 __global__ void k_avbd_warmstart(const DevState d, Params p, int cur) {
@@ -1105,6 +1114,10 @@ __global__ void k_avbd_warmstart(const DevState d, Params p, int cur) {
     Quatf q1c = q_conj(d1 ? q_from(d.a_rot_start[b.x]) : q_from(d.rot[b.x]));
     Quatf q2c = q_conj(d2 ? q_from(d.a_rot_start[b.y]) : q_from(d.rot[b.y]));
     const int cc = d.m_keycc[cur][slot].y;
+    const float3 td[2] = {f3(d.m_t0[cur][slot]), f3(d.m_t1[cur][slot])};
+    const float mu = sqrtf(fmaxf(d.iinv[b.x].w, 0.f) * fmaxf(d.iinv[b.y].w, 0.f));
+    const Quatf q1 = d1 ? q_from(d.a_rot_start[b.x]) : q_from(d.rot[b.x]);
+    const Quatf q2 = d2 ? q_from(d.a_rot_start[b.y]) : q_from(d.rot[b.y]);
     uint32_t sticks = 0;
     for (int j = 0; j < cc; ++j) {
       const uint32_t ci = slot * BB_MAX_CONTACTS + j;
@@ -1123,16 +1136,25 @@ __global__ void k_avbd_warmstart(const DevState d, Params p, int cur) {
         kt.y = fminf(fmaxf(kt.y * p.avbd_gamma, p.avbd_k_min), p.avbd_k_max);
       }
       bool sticking = matched && stick != 0u;
+      const float4 cp = d.c_pos[cur][ci];
+      float4 aa = d.c_anc_a[cur][ci], ab = d.c_anc_b[cur][ci];
       if (!sticking) {
-        float4 cp = d.c_pos[cur][ci];
-        float4 aa = d.c_anc_a[cur][ci];
-        d.c_anc_a[cur][ci] = f4(avbd_q_rotate(q1c, f3(cp) - c1), aa.w);
-        d.c_anc_b[cur][ci] = f4(avbd_q_rotate(q2c, f3(cp) - c2), 0.f);
+        aa = f4(avbd_q_rotate(q1c, f3(cp) - c1), aa.w);
+        ab = f4(avbd_q_rotate(q2c, f3(cp) - c2), 0.f);
+        d.c_anc_a[cur][ci] = aa;
+        d.c_anc_b[cur][ci] = ab;
       } else {
         ++sticks;
       }
       d.c_lam[cur][ci] = lam;
       d.c_kt[cur][ci] = make_float4(kt.x, kt.y, __uint_as_float(stick), kt.w);
+      // rows: what the sweeps need of this contact that no sweep changes
+      const float3 ar1 = avbd_q_rotate(q1, f3(aa)), ar2 = avbd_q_rotate(q2, f3(ab));
+      const float3 sep = (c2 + ar2) - (c1 + ar1);
+      d.c_r1[ci] = f4(f3(cp) - c1, cp.w + p.avbd_margin);
+      d.c_r2[ci] = f4(f3(cp) - c2, dot3(td[0], sep));
+      d.c_k[ci] = f4(ar1, dot3(td[1], sep));
+      d.pgs_lam[ci] = f4(ar2, mu);
     }
     if (sticks) atomicAdd(&d.ctr->stick, sticks);
   }
@@ -1155,8 +1177,82 @@ __global__ void k_avbd_depth_relax(const DevState d, int cur) {
   }
 }
 
-// bucket keys of awake coloured bodies: pass 0 = colour (main sweeps),
-// pass 1 = min(depth, L-1) * 32 + colour (post-stabilisation cascade); others sort last
+// starts[v] = first sorted position with key >= v * scale, for v in [0, nb]
+__global__ void k_lower_bounds(const uint32_t* keys, uint32_t n, uint32_t* starts, uint32_t nb, uint32_t scale) {
+  uint32_t v = blockIdx.x * blockDim.x + threadIdx.x;
+  if (v > nb) return;
+  uint32_t lo = 0, hi = n;
+  while (lo < hi) {
+    uint32_t mid = (lo + hi) >> 1;
+    if (keys[mid] < v * scale) lo = mid + 1;
+    else hi = mid;
+  }
+  starts[v] = lo;
+}
+
+// One contact's rows, written once per substep by k_avbd_warmstart at the contact's slot index:
+// R0 = lever arm on a and depth + margin, R1 = lever arm on b and the start separation along
+// tangent 0, R2 = anchor arm on a and the separation along tangent 1, R3 = anchor arm on b and
+// the pair's friction.  The sweeps visit a contact some 25 times per body and substep; forming
+// these from positions, start poses and anchors on each visit took ~20 dependent gathers.
+struct AvbdRow {
+  float4 r0, r1, r2, r3;
+};
+__device__ __forceinline__ AvbdRow avbd_row(const DevState& d, uint32_t ci) {
+  return AvbdRow{d.c_r1[ci], d.c_r2[ci], d.c_k[ci], d.pgs_lam[ci]};
+}
+// displacements of a manifold's two bodies since the step's start
+struct AvbdDisp {
+  float3 dp1, dth1, dp2, dth2;
+};
+
+__device__ __forceinline__ float avbd_contact_C(const AvbdRow& r, const AvbdDisp& u, bool d1, bool d2, float alpha, float3 n) {
+  float C = r.r0.w * (1.0f - alpha);
+  if (d1) C -= dot3(n, u.dp1 + cross3(u.dth1, f3(r.r0)));
+  if (d2) C += dot3(n, u.dp2 + cross3(u.dth2, f3(r.r1)));
+  return C;
+}
+
+__device__ __forceinline__ float avbd_dir_C(const AvbdRow& r, const AvbdDisp& u, float C0t, float slop, bool d1, bool d2,
+                                            float alpha, float3 dir) {
+  float sg = C0t > 0.f ? 1.f : (C0t < 0.f ? -1.f : 0.f);
+  float c0e = sg * fmaxf(0.f, fabsf(C0t) - slop);
+  float C = c0e * (1.0f - alpha);
+  if (d1) C -= dot3(dir, u.dp1 + cross3(u.dth1, f3(r.r2)));
+  if (d2) C += dot3(dir, u.dp2 + cross3(u.dth2, f3(r.r3)));
+  return C;
+}
+
+// per entry of the bodies' manifold lists: x = partner | partner awake << 30 | this body is a << 31,
+// y = slot | (contact count - 1) << 29
+__device__ __forceinline__ uint2* avbd_entries(const DevState& d) { return reinterpret_cast<uint2*>(d.pgs_rec); }
+__device__ __forceinline__ uint32_t* avbd_class(const DevState& d) { return d.flow_counter; }
+// Also the body's work class, 0 for the most: by the contacts of its longest lane (lane l sums the
+// manifolds l, l + AVBD_LANES, ... of the list).  The sweeps take a colour's bodies by class, so
+// that the bodies of a warp are equally long and the long ones start first.
+#define AVBD_LANES 8
+#define AVBD_CLASSES 7u
+__global__ void k_avbd_entries(const DevState d, uint32_t n, int cur) {
+  const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= n || !awake(d.flags[i])) return;
+  uint32_t len[AVBD_LANES] = {}, l = 0, most = 0;
+  for (uint32_t e = d.csr_start[cur][i]; e < d.csr_start[cur][i + 1]; ++e, l = (l + 1) % AVBD_LANES) {
+    const uint32_t slot = d.csr_slot[cur][e], q = d.csr_partner[cur][e], cc = uint32_t(d.m_keycc[cur][slot].y);
+    avbd_entries(d)[e] = make_uint2(q | (awake(d.flags[q]) ? 1u << 30 : 0u) | (d.m_bodies[cur][slot].x == i ? 1u << 31 : 0u),
+                                    slot | (cc - 1u) << 29);
+#pragma unroll
+    for (int k = 0; k < AVBD_LANES; ++k)
+      if (uint32_t(k) == l) {
+        len[k] += cc;
+        most = max(most, len[k]);
+      }
+  }
+  avbd_class(d)[i] = most > 8u ? 0u : most > 6u ? 1u : most > 4u ? 2u : most > 3u ? 3u : most > 2u ? 4u : most > 1u ? 5u : 6u;
+}
+
+// bucket keys of awake coloured bodies: bucket * AVBD_CLASSES + work class, where the bucket is the
+// colour (main and last sweeps) or min(depth, L-1) * 32 + colour (post-stabilisation cascade);
+// others sort last
 __global__ void k_avbd_keys(const DevState d, Params p, uint32_t n, int post) {
   uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
@@ -1169,89 +1265,32 @@ __global__ void k_avbd_keys(const DevState d, Params p, uint32_t n, int post) {
     } else {
       key = col;
     }
+    key = key * AVBD_CLASSES + avbd_class(d)[i];
   }
   d.a_bucket_keys[0][i] = key;
   d.a_bucket_vals[0][i] = i;
 }
-// starts[v] = first sorted position with key >= v, for v in [0, nb]
-__global__ void k_lower_bounds(const uint32_t* keys, uint32_t n, uint32_t* starts, uint32_t nb) {
-  uint32_t v = blockIdx.x * blockDim.x + threadIdx.x;
-  if (v > nb) return;
-  uint32_t lo = 0, hi = n;
-  while (lo < hi) {
-    uint32_t mid = (lo + hi) >> 1;
-    if (keys[mid] < v) lo = mid + 1;
-    else hi = mid;
-  }
-  starts[v] = lo;
-}
-
-struct AvbdCtx {
-  float dt;
-};
-
-__device__ float avbd_contact_C(const DevState& d, const Params& p, int cur, uint32_t slot, uint32_t ci, uint2 b,
-                                bool d1, bool d2, float alpha, float3 n, float3& rr1, float3& rr2) {
-  float4 cp = d.c_pos[cur][ci];
-  float3 c1 = d1 ? f3(d.a_pos_start[b.x]) : f3(d.pos[b.x]);
-  float3 c2 = d2 ? f3(d.a_pos_start[b.y]) : f3(d.pos[b.y]);
-  rr1 = f3(cp) - c1;
-  rr2 = f3(cp) - c2;
-  float C = (cp.w + p.avbd_margin) * (1.0f - alpha);
-  if (d1) {
-    float3 dp = f3(d.pos[b.x]) - c1;
-    float3 dth = small_angle_delta(q_from(d.rot[b.x]), q_from(d.a_rot_start[b.x]));
-    C -= dot3(n, dp + cross3(dth, rr1));
-  }
-  if (d2) {
-    float3 dp = f3(d.pos[b.y]) - c2;
-    float3 dth = small_angle_delta(q_from(d.rot[b.y]), q_from(d.a_rot_start[b.y]));
-    C += dot3(n, dp + cross3(dth, rr2));
-  }
-  (void)slot;
-  return C;
-}
-
-__device__ float avbd_dir_C(const DevState& d, const Params& p, int cur, uint32_t ci, uint2 b, bool d1, bool d2,
-                            float alpha, float3 dir, float3& ar1, float3& ar2, float& C0t) {
-  float3 c1 = d1 ? f3(d.a_pos_start[b.x]) : f3(d.pos[b.x]);
-  float3 c2 = d2 ? f3(d.a_pos_start[b.y]) : f3(d.pos[b.y]);
-  Quatf q1 = d1 ? q_from(d.a_rot_start[b.x]) : q_from(d.rot[b.x]);
-  Quatf q2 = d2 ? q_from(d.a_rot_start[b.y]) : q_from(d.rot[b.y]);
-  ar1 = avbd_q_rotate(q1, f3(d.c_anc_a[cur][ci]));
-  ar2 = avbd_q_rotate(q2, f3(d.c_anc_b[cur][ci]));
-  C0t = dot3(dir, (c2 + ar2) - (c1 + ar1));
-  float sg = C0t > 0.f ? 1.f : (C0t < 0.f ? -1.f : 0.f);
-  float c0e = sg * fmaxf(0.f, fabsf(C0t) - p.avbd_stick_slop);
-  float C = c0e * (1.0f - alpha);
-  if (d1) {
-    float3 dp = f3(d.pos[b.x]) - c1;
-    float3 dth = small_angle_delta(q_from(d.rot[b.x]), q_from(d.a_rot_start[b.x]));
-    C -= dot3(dir, dp + cross3(dth, ar1));
-  }
-  if (d2) {
-    float3 dp = f3(d.pos[b.y]) - c2;
-    float3 dth = small_angle_delta(q_from(d.rot[b.y]), q_from(d.a_rot_start[b.y]));
-    C += dot3(dir, dp + cross3(dth, ar2));
-  }
-  return C;
-}
-
-// entry_avbd_primal (avbd.slang:478-658): Gauss-Newton step of body i on its 6 DoF.
+// entry_avbd_primal (avbd.slang:478-658): Gauss-Newton step of body i on its 6 DoF, in two
+// parts: the sums over its contacts (avbd_gather) and the solve (avbd_move).
 // A group of AVBD_LANES lanes per body.  Lane l of the group takes manifolds l, l + AVBD_LANES, ...
 // of the body's list and sums their contacts' gradient and Hessian terms in order; a butterfly
 // over the group adds the lanes' sums (a fixed order, so the result does not depend on
-// scheduling or on which bodies share a warp; it differs from a serial sum in the last bits),
-// and the group's lane 0 adds the inertial terms, solves the 6x6 system and moves the body.
+// scheduling or on which bodies share a warp; it differs from a serial sum in the last bits);
+// one lane then adds the inertial terms, solves the 6x6 system and moves the body.
 // Serially, a body's whole contact loop was one dependent chain per colour step (a box in a
 // pile: 15-30 us); a warp per body cut the chain but left too few bodies in flight where a
 // colour holds tens of thousands of them.  i == BB_NONE: the group only takes part in the
-// shuffles (the trips over a colour's bodies are warp-uniform).
+// shuffles (the trips over a colour's bodies are block-uniform).
+// Bound: latency, the contacts of a colour's longest bodies one after the other, 100 to 250 dependent
+// colour steps per substep.  Solve stage per substep, with poses and anchors gathered per visit
+// and the solve on one lane in eight of 512-thread blocks -> now: 8.3 -> 3.3 ms on a 20k mixed
+// pile (10 iterations), 6.9 -> 4.0 ms on 256 batched worlds (119k bodies, 4 iterations).  Tried and
+// slower: the next contact's rows loaded, prefetched to L1 or staged by cp.async ahead of use.
 // H is kept as its lower triangle, row-major: entry (a, b), b <= a, at a * (a + 1) / 2 + b.
-#define AVBD_LANES 8
-#define AVBD_GROUPS (32 / AVBD_LANES)
+#define AVBD_THREADS 128  // small blocks: a world of few bodies spreads over more SMs
+#define AVBD_BODIES (AVBD_THREADS / AVBD_LANES)  // bodies of a block's trip
 __device__ __forceinline__ int avbd_lt(int a, int b) { return a * (a + 1) / 2 + b; }
-__device__ __forceinline__ void avbd_primal(const DevState& d, const Params& p, int cur, uint32_t i, float dt, float alpha) {
+__device__ __forceinline__ void avbd_gather(const DevState& d, const Params& p, int cur, uint32_t i, float alpha, float* out) {
   const int lane = threadIdx.x & (AVBD_LANES - 1);
   float g[6], H[21];
 #pragma unroll
@@ -1259,24 +1298,35 @@ __device__ __forceinline__ void avbd_primal(const DevState& d, const Params& p, 
 #pragma unroll
   for (int a = 0; a < 21; ++a) H[a] = 0.f;
   const uint32_t s0 = i == BB_NONE ? 0u : d.csr_start[cur][i], s1 = i == BB_NONE ? 0u : d.csr_start[cur][i + 1];
+  float3 odp{}, odth{};
+  if (i != BB_NONE) {
+    odp = f3(d.iw[2 * size_t(i)]);
+    odth = f3(d.iw[2 * size_t(i) + 1]);
+  }
   for (uint32_t e = s0 + uint32_t(lane); e < s1; e += AVBD_LANES) {
-    const uint32_t slot = d.man_slot[cur][d.csr_list[cur][e]];
-    const int cc = d.m_keycc[cur][slot].y;
-    const uint2 b = d.m_bodies[cur][slot];
-    const bool i1 = b.x == i;
-    const bool d1 = awake(d.flags[b.x]), d2 = awake(d.flags[b.y]);
-    const float mu = sqrtf(fmaxf(d.iinv[b.x].w, 0.f) * fmaxf(d.iinv[b.y].w, 0.f));
+    const uint2 en = avbd_entries(d)[e];
+    const bool i1 = en.x >> 31, qa = (en.x >> 30) & 1u;
+    const uint32_t q = en.x & 0x3FFFFFFFu, slot = en.y & 0x1FFFFFFFu;
+    const int cc = int(en.y >> 29) + 1;
+    const bool d1 = i1 || qa, d2 = !i1 || qa;
     const float3 n = f3(d.m_normal[cur][slot]);
     const float3 td[2] = {f3(d.m_t0[cur][slot]), f3(d.m_t1[cur][slot])};
+    float3 qdp{}, qdth{};
+    if (qa) {
+      qdp = f3(d.iw[2 * size_t(q)]);
+      qdth = f3(d.iw[2 * size_t(q) + 1]);
+    }
+    const AvbdDisp u = i1 ? AvbdDisp{odp, odth, qdp, qdth} : AvbdDisp{qdp, qdth, odp, odth};
     for (int j = 0; j < cc; ++j) {
       const uint32_t ci = slot * BB_MAX_CONTACTS + uint32_t(j);
-      float3 rr1, rr2;
-      const float C = avbd_contact_C(d, p, cur, slot, ci, b, d1, d2, alpha, n, rr1, rr2);
+      const AvbdRow r = avbd_row(d, ci);
       const float4 lam = d.c_lam[cur][ci];
       const float4 kt = d.c_kt[cur][ci];
+      const float mu = r.r3.w;
+      const float C = avbd_contact_C(r, u, d1, d2, alpha, n);
       const float f = fminf(lam.w * C + lam.x, 0.f);
       const float3 Jl = i1 ? -n : n;
-      const float3 Ja = i1 ? -cross3(rr1, n) : cross3(rr2, n);
+      const float3 Ja = i1 ? -cross3(f3(r.r0), n) : cross3(f3(r.r1), n);
       const float J[6] = {Jl.x, Jl.y, Jl.z, Ja.x, Ja.y, Ja.z};
 #pragma unroll
       for (int a = 0; a < 6; ++a) g[a] += f * J[a];
@@ -1287,14 +1337,12 @@ __device__ __forceinline__ void avbd_primal(const DevState& d, const Params& p, 
       const float bound = mu * fabsf(lam.x);
 #pragma unroll
       for (int t = 0; t < 2; ++t) {
-        float3 ar1, ar2;
-        float C0t;
-        const float Ct = avbd_dir_C(d, p, cur, ci, b, d1, d2, alpha, td[t], ar1, ar2, C0t);
+        const float Ct = avbd_dir_C(r, u, t == 0 ? r.r1.w : r.r2.w, p.avbd_stick_slop, d1, d2, alpha, td[t]);
         const float ktt = t == 0 ? kt.x : kt.y;
         const float lt = t == 0 ? lam.y : lam.z;
         const float ft = fminf(fmaxf(ktt * Ct + lt, -bound), bound);
         const float3 Jlt = i1 ? -td[t] : td[t];
-        const float3 Jat = i1 ? -cross3(ar1, td[t]) : cross3(ar2, td[t]);
+        const float3 Jat = i1 ? -cross3(f3(r.r2), td[t]) : cross3(f3(r.r3), td[t]);
         const float Jt[6] = {Jlt.x, Jlt.y, Jlt.z, Jat.x, Jat.y, Jat.z};
 #pragma unroll
         for (int a = 0; a < 6; ++a) g[a] += ft * Jt[a];
@@ -1313,6 +1361,19 @@ __device__ __forceinline__ void avbd_primal(const DevState& d, const Params& p, 
     for (int a = 0; a < 21; ++a) H[a] += __shfl_xor_sync(0xFFFFFFFFu, H[a], o);
   }
   if (lane != 0 || i == BB_NONE) return;
+#pragma unroll
+  for (int a = 0; a < 6; ++a) out[a * AVBD_BODIES] = g[a];
+#pragma unroll
+  for (int a = 0; a < 21; ++a) out[(6 + a) * AVBD_BODIES] = H[a];
+}
+
+// the step of body i from its summed gradient and Hessian: inertial terms, 6x6 solve, new pose
+__device__ __forceinline__ void avbd_move(const DevState& d, const Params& p, uint32_t i, float dt, const float* sum) {
+  float g[6], H[21];
+#pragma unroll
+  for (int a = 0; a < 6; ++a) g[a] = sum[a * AVBD_BODIES];
+#pragma unroll
+  for (int a = 0; a < 21; ++a) H[a] = sum[(6 + a) * AVBD_BODIES];
   const bool tq = p.quirks & BB_QUIRK_INERTIA_TRANSPOSE;
   const float inv_dt2 = dt > 0.f ? 1.0f / (dt * dt) : 0.f;
   const float m_lin = d.vel[i].w * inv_dt2;
@@ -1386,26 +1447,41 @@ __device__ __forceinline__ void avbd_primal(const DevState& d, const Params& p, 
       if (kk > ii) sm -= H[avbd_lt(kk, ii)] * x[kk];
     x[ii] = sm;
   }
-  float4 ps = d.pos[i];
-  d.pos[i] = make_float4(ps.x + x[0], ps.y + x[1], ps.z + x[2], ps.w);
+  const float4 ps = d.pos[i];
+  const float3 pn = make_float3(ps.x + x[0], ps.y + x[1], ps.z + x[2]);
+  d.pos[i] = f4(pn, ps.w);
   Quatf dq{x[3] * 0.5f, x[4] * 0.5f, x[5] * 0.5f, 1.0f};
-  d.rot[i] = q_to4(q_normalize(q_mul(dq, rot)));
+  const Quatf qn = q_normalize(q_mul(dq, rot));
+  d.rot[i] = q_to4(qn);
+  avbd_store_disp(d, i, pn - f3(d.a_pos_start[i]), small_angle_delta(qn, q_from(d.a_rot_start[i])));
 }
 
 // entry_avbd_dual (avbd.slang:728-808)
-__device__ void avbd_dual(const DevState& d, const Params& p, int cur, uint32_t m) {
+// lane l of a manifold's AVBD_DUAL_LANES lanes takes contacts l, l + AVBD_DUAL_LANES, ... (they are
+// independent): neighbouring lanes read neighbouring 16 bytes of each plane
+#define AVBD_DUAL_LANES 4
+__device__ void avbd_dual(const DevState& d, const Params& p, int cur, uint32_t m, int lane) {
   const uint32_t slot = d.man_slot[cur][m];
   const uint2 b = d.m_bodies[cur][slot];
   const bool d1 = awake(d.flags[b.x]), d2 = awake(d.flags[b.y]);
   if (!d1 && !d2) return;
-  const float mu = sqrtf(fmaxf(d.iinv[b.x].w, 0.f) * fmaxf(d.iinv[b.y].w, 0.f));
   const float3 n = f3(d.m_normal[cur][slot]);
   const float3 td[2] = {f3(d.m_t0[cur][slot]), f3(d.m_t1[cur][slot])};
   const int cc = d.m_keycc[cur][slot].y;
-  for (int j = 0; j < cc; ++j) {
+  AvbdDisp u{};
+  if (d1) {
+    u.dp1 = f3(d.iw[2 * size_t(b.x)]);
+    u.dth1 = f3(d.iw[2 * size_t(b.x) + 1]);
+  }
+  if (d2) {
+    u.dp2 = f3(d.iw[2 * size_t(b.y)]);
+    u.dth2 = f3(d.iw[2 * size_t(b.y) + 1]);
+  }
+  for (int j = lane; j < cc; j += AVBD_DUAL_LANES) {
     const uint32_t ci = slot * BB_MAX_CONTACTS + j;
-    float3 rr1, rr2;
-    float C = avbd_contact_C(d, p, cur, slot, ci, b, d1, d2, 1.0f, n, rr1, rr2);
+    const AvbdRow r = avbd_row(d, ci);
+    const float mu = r.r3.w;
+    const float C = avbd_contact_C(r, u, d1, d2, 1.0f, n);
     float4 lam = d.c_lam[cur][ci];
     float4 kt = d.c_kt[cur][ci];
     const float lam0 = lam.x, k = lam.w;
@@ -1417,9 +1493,8 @@ __device__ void avbd_dual(const DevState& d, const Params& p, int cur, uint32_t 
     float drift2 = 0.f;
 #pragma unroll
     for (int t = 0; t < 2; ++t) {
-      float3 ar1, ar2;
-      float C0t;
-      float Ct = avbd_dir_C(d, p, cur, ci, b, d1, d2, 1.0f, td[t], ar1, ar2, C0t);
+      const float C0t = t == 0 ? r.r1.w : r.r2.w;
+      const float Ct = avbd_dir_C(r, u, C0t, p.avbd_stick_slop, d1, d2, 1.0f, td[t]);
       float lt = t == 0 ? lam.y : lam.z;
       float ktt = t == 0 ? kt.x : kt.y;
       float nlt = fminf(fmaxf(ktt * Ct + lt, -bound), bound);
@@ -1457,52 +1532,69 @@ __device__ void avbd_finalize(const DevState& d, int cur, uint32_t i, float dt) 
   d.omega[i] = f4(w, 0.f);
 }
 
-// persistent solve: main iterations (colour sweeps + dual), finalize, post-stabilisation
-__global__ void __launch_bounds__(BB_COOP_THREADS, 1) k_avbd_solve(const DevState d, Params p, int cur, uint32_t n, float dt,
-                                                           int phase) {
-  const uint32_t tid = blockIdx.x * blockDim.x + threadIdx.x, stride = gridDim.x * blockDim.x;
-  // primal sweeps: AVBD_GROUPS bodies per warp (AVBD_LANES lanes each), warp-uniform trips
-  const uint32_t wid = tid >> 5, nwarps = stride >> 5, grp = (threadIdx.x & 31u) / AVBD_LANES;
+// One bucket of bodies, no two of which share a manifold: a block takes AVBD_BODIES of them per
+// trip.  All lanes sum the contacts; then the block's first lanes solve one body each, so that
+// the 6x6 solve (hundreds of instructions) is issued once per block and trip and not by every warp
+// for its few bodies.  buf alternates, so a trip's sums are written while the last one's are solved.
+__device__ __forceinline__ void avbd_bucket(const DevState& d, const Params& p, int cur, uint32_t s0, uint32_t s1, float dt,
+                                            float alpha, float* sums, uint32_t& trip) {
   const uint32_t* list = d.a_bucket_vals[1];
+  for (uint32_t base = s0 + blockIdx.x * AVBD_BODIES; base < s1; base += gridDim.x * AVBD_BODIES, ++trip) {
+    float* buf = sums + (trip & 1u) * 27 * AVBD_BODIES;
+    const uint32_t k = base + threadIdx.x / AVBD_LANES;
+    const bool mover = threadIdx.x < AVBD_BODIES && base + threadIdx.x < s1;
+    const uint32_t mine = mover ? list[base + threadIdx.x] : 0u;
+    avbd_gather(d, p, cur, k < s1 ? list[k] : BB_NONE, alpha, buf + threadIdx.x / AVBD_LANES);
+    __syncthreads();
+    if (mover) avbd_move(d, p, mine, dt, buf + threadIdx.x);
+  }
+}
+
+// persistent solve: main iterations (colour sweeps + dual), finalize, post-stabilisation
+__global__ void __launch_bounds__(AVBD_THREADS, 512 / AVBD_THREADS) k_avbd_solve(const DevState d, Params p, int cur,
+                                                                                 uint32_t n, float dt, int phase) {
+  __shared__ float sums[2 * 27 * AVBD_BODIES];
+  __shared__ uint32_t bs[64 * BB_MAX_COLORS + 1];  // starts of the buckets that hold bodies, and their end
+  __shared__ uint32_t s_nb;
+  const uint32_t tid = blockIdx.x * blockDim.x + threadIdx.x, stride = gridDim.x * blockDim.x;
   uint32_t* sync = &d.ctr->sync_count[3 + phase];
-  uint32_t ep = 0;
-  if (phase == 0) {
-    const uint32_t C = d.ctr->avbd_colors;
-    const uint32_t M = d.ctr->manifold_count;
-    for (uint32_t it = 0; it < p.avbd_iterations; ++it) {
-      for (uint32_t c = 0; c < C; ++c) {
-        uint32_t s0 = d.a_bucket_start[c], s1 = d.a_bucket_start[c + 1];
-        if (s0 == s1) continue;
-        for (uint32_t kw = s0 + wid * AVBD_GROUPS; kw < s1; kw += nwarps * AVBD_GROUPS)
-          avbd_primal(d, p, cur, kw + grp < s1 ? list[kw + grp] : BB_NONE, dt, 1.0f);
-        grid_sync(d.ctr, sync, ep);
-      }
-      for (uint32_t m = tid; m < M; m += stride) avbd_dual(d, p, cur, m);
-      grid_sync(d.ctr, sync, ep);
+  uint32_t ep = 0, trip = 0;
+  const uint32_t keys = phase == 1 ? p.avbd_shock_layers * BB_MAX_COLORS : min(d.ctr->avbd_colors, uint32_t(BB_MAX_COLORS));
+  if (threadIdx.x < 32u) {
+    uint32_t c = 0;
+    for (uint32_t k0 = 0; k0 < keys; k0 += 32u) {
+      const uint32_t k = k0 + threadIdx.x;
+      const uint32_t a = k < keys ? d.a_bucket_start[k] : 0u;
+      const bool full = k < keys && d.a_bucket_start[k + 1] != a;
+      const uint32_t m = __ballot_sync(0xFFFFFFFFu, full);
+      if (full) bs[c + uint32_t(__popc(m & ((1u << threadIdx.x) - 1u)))] = a;
+      c += uint32_t(__popc(m));
     }
-    for (uint32_t i = tid; i < n; i += stride)
-      if (awake(d.flags[i])) avbd_finalize(d, cur, i, dt);
-  } else if (phase == 1) {
-    const uint32_t nb = p.avbd_shock_layers * BB_MAX_COLORS;
-    for (uint32_t key = 0; key < nb; ++key) {
-      uint32_t s0 = d.a_bucket_start[key], s1 = d.a_bucket_start[key + 1];
-      if (s0 == s1) continue;
-      for (uint32_t kw = s0 + wid * AVBD_GROUPS; kw < s1; kw += nwarps * AVBD_GROUPS)
-        avbd_primal(d, p, cur, kw + grp < s1 ? list[kw + grp] : BB_NONE, dt, 0.0f);
-      grid_sync(d.ctr, sync, ep);
-    }
-  } else {
-    const uint32_t C = d.ctr->avbd_colors;
-    for (uint32_t sw = 1; sw < p.avbd_post_stab_sweeps; ++sw) {
-      for (uint32_t c = 0; c < C; ++c) {
-        uint32_t s0 = d.a_bucket_start[c], s1 = d.a_bucket_start[c + 1];
-        if (s0 == s1) continue;
-        for (uint32_t kw = s0 + wid * AVBD_GROUPS; kw < s1; kw += nwarps * AVBD_GROUPS)
-          avbd_primal(d, p, cur, kw + grp < s1 ? list[kw + grp] : BB_NONE, dt, 0.0f);
-        grid_sync(d.ctr, sync, ep);
-      }
+    if (threadIdx.x == 0) {
+      bs[c] = keys ? d.a_bucket_start[keys] : 0u;
+      s_nb = c;
     }
   }
+  __syncthreads();
+  const uint32_t nb = s_nb;
+  // sweeps over the buckets, a barrier after each; after each of the main iterations the dual step
+  const uint32_t sweeps = phase == 0 ? p.avbd_iterations : phase == 1 ? 1u : p.avbd_post_stab_sweeps - 1u;
+  const float alpha = phase == 0 ? 1.0f : 0.0f;
+  const uint32_t M = d.ctr->manifold_count;
+  for (uint32_t sw = 0; sw < sweeps; ++sw) {
+    for (uint32_t b = 0; b < nb; ++b) {
+      avbd_bucket(d, p, cur, bs[b], bs[b + 1], dt, alpha, sums, trip);
+      grid_sync(d.ctr, sync, ep);
+    }
+    if (phase == 0) {
+      for (uint32_t m = tid / AVBD_DUAL_LANES; m < M; m += stride / AVBD_DUAL_LANES)
+        avbd_dual(d, p, cur, m, int(threadIdx.x % AVBD_DUAL_LANES));
+      grid_sync(d.ctr, sync, ep);
+    }
+  }
+  if (phase == 0)
+    for (uint32_t i = tid; i < n; i += stride)
+      if (awake(d.flags[i])) avbd_finalize(d, cur, i, dt);
 }
 
 // Scratch of the body bucket sorts (every region is zeroed once per substep and used once):
@@ -1515,21 +1607,27 @@ static void avbd_buckets(cudaStream_t s, const DevState& d, const Params& p, uin
   uint32_t* keys[2] = {d.a_bucket_keys[0], d.a_bucket_keys[1]};
   uint32_t* vals[2] = {d.a_bucket_vals[0], d.a_bucket_vals[1]};
   uint32_t* hist = sc.sort_hist + size_t(region) * BB_HIST_REGION;
-  // post keys need 9 bits; three 8-bit passes (the third sees only zero digits, so it keeps
+  // post keys need up to 14 bits; three 8-bit passes (the third sees only zero digits, so it keeps
   // the order) leave the result in buffer 1 like the one-pass colour sort
   bb_launch_sort(s, keys, vals, nullptr, n, post ? 3 : 1, 0, hist, sc.sort_status + size_t(slot) * sc.sort_tiles * 256,
                  sc.sort_tile_ctr + slot, d.ctr, sms);
   uint32_t nb = post ? p.avbd_shock_layers * BB_MAX_COLORS : BB_MAX_COLORS;
-  k_lower_bounds<<<(nb + 1 + 127) / 128, 128, 0, s>>>(d.a_bucket_keys[1], n, d.a_bucket_start, nb);
+  k_lower_bounds<<<(nb + 1 + 127) / 128, 128, 0, s>>>(d.a_bucket_keys[1], n, d.a_bucket_start, nb, AVBD_CLASSES);
 }
 
-int bb_avbd_blocks(int sms) {
-  return std::min(bb_coop_blocks((const void*)k_avbd_color, BB_COOP_THREADS, sms),
-                  bb_coop_blocks((const void*)k_avbd_solve, BB_COOP_THREADS, sms));
+int bb_avbd_color_blocks(int sms) { return bb_coop_blocks((const void*)k_avbd_color, BB_COOP_THREADS, sms); }
+// Blocks of k_avbd_solve: AVBD_THREADS threads, 512 per SM in all; for a world of n bodies as many
+// as hold one thread per body (8 lanes for each body of the largest colour, about an eighth)
+int bb_avbd_blocks(int sms, uint32_t max_bodies) {
+  int per_sm = 0;
+  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, (const void*)k_avbd_solve, AVBD_THREADS, 0);
+  per_sm = std::max(1, std::min(per_sm, 512 / AVBD_THREADS));
+  const uint64_t want = (uint64_t(max_bodies) + AVBD_THREADS - 1) / AVBD_THREADS;
+  return int(std::max<uint64_t>(1, std::min<uint64_t>(uint64_t(sms) * per_sm, want)));
 }
 
 void bb_solve_avbd(cudaStream_t s, const DevState& d, const Params& p, uint32_t n, float h, const StepScratch& sc,
-                   int sms, int cur, int coop_blocks) {
+                   int sms, int cur, int coop_blocks, int color_blocks) {
   if (n == 0) return;
   const int T = BB_THREADS;
   uint32_t blocks = (n + T - 1) / T;
@@ -1539,10 +1637,11 @@ void bb_solve_avbd(cudaStream_t s, const DevState& d, const Params& p, uint32_t 
     int cc = cur;
     uint32_t nn = n;
     void* args[] = {&dd, &pp, &cc, &nn};
-    bb_launch_coop((const void*)k_avbd_color, coop_blocks, BB_COOP_THREADS, args, s);
+    bb_launch_coop((const void*)k_avbd_color, color_blocks, BB_COOP_THREADS, args, s);
   }
   k_avbd_prepare<<<blocks, T, 0, s>>>(d, p, n, h);
   k_avbd_warmstart<<<sms * 8, T, 0, s>>>(d, p, cur);
+  k_avbd_entries<<<blocks, T, 0, s>>>(d, n, cur);
   k_avbd_depth_reset<<<blocks, T, 0, s>>>(d, n);
   for (uint32_t k = 0; k < p.avbd_shock_layers; ++k) k_avbd_depth_relax<<<sms * 8, T, 0, s>>>(d, cur);
   DevState dd = d;
@@ -1553,15 +1652,15 @@ void bb_solve_avbd(cudaStream_t s, const DevState& d, const Params& p, uint32_t 
   int phase = 0;
   void* args[] = {&dd, &pp, &cc, &nn, &hh, &phase};
   avbd_buckets(s, d, p, n, sc, sms, 0, 2, 7);
-  bb_launch_coop((const void*)k_avbd_solve, coop_blocks, BB_COOP_THREADS, args, s);
+  bb_launch_coop((const void*)k_avbd_solve, coop_blocks, AVBD_THREADS, args, s);
   avbd_buckets(s, d, p, n, sc, sms, 1, 3, 8);  // slots 8, 9, 10
   int phase1 = 1;
   void* args1[] = {&dd, &pp, &cc, &nn, &hh, &phase1};
-  bb_launch_coop((const void*)k_avbd_solve, coop_blocks, BB_COOP_THREADS, args1, s);
+  bb_launch_coop((const void*)k_avbd_solve, coop_blocks, AVBD_THREADS, args1, s);
   if (p.avbd_post_stab_sweeps > 1) {
     avbd_buckets(s, d, p, n, sc, sms, 0, 4, 11);
     int phase2 = 2;
     void* args2[] = {&dd, &pp, &cc, &nn, &hh, &phase2};
-    bb_launch_coop((const void*)k_avbd_solve, coop_blocks, BB_COOP_THREADS, args2, s);
+    bb_launch_coop((const void*)k_avbd_solve, coop_blocks, AVBD_THREADS, args2, s);
   }
 }

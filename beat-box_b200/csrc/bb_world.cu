@@ -355,7 +355,7 @@ struct bb_world_impl {
   int last_cur = 0;  // manifold buffer the last (partial or full) substep wrote
   bool skip_warm_once = false;
   bool ran_any = false;
-  int coop_edge = 0, coop_pgs = 0, coop_avbd = 0, coop_cc = 0;
+  int coop_edge = 0, coop_pgs = 0, coop_avbd = 0, coop_avbd_color = 0, coop_cc = 0;
   size_t scratch_bytes = 0;
   void* scratch_base = nullptr;
   size_t dev_bytes = 0;  // device memory held by this world
@@ -649,7 +649,7 @@ struct bb_world_impl {
     bb_sleep(stream, d, params, n, sms, cur);
     const bool coloured = (params.flags & BB_SIM_USE_GRAPH_COLORING) != 0;
     if (coloured || params.solver == BB_SOLVER_AVBD) bb_edge_coloring(stream, d, params, n, sc, sms, cur, coop_edge);
-    if (params.solver == BB_SOLVER_AVBD) bb_solve_avbd(stream, d, params, n, h, sc, sms, cur, coop_avbd);
+    if (params.solver == BB_SOLVER_AVBD) bb_solve_avbd(stream, d, params, n, h, sc, sms, cur, coop_avbd, coop_avbd_color);
     else if (!coloured) bb_solve_islands(stream, d, params, n, h, cur, sc, sms);
     else bb_solve_pgs_soft(stream, d, params, n, h, cur, sc, coop_pgs, sms);
     if (commit) parity = cur;
@@ -767,7 +767,8 @@ bb_status bb_world_create(const bb_world_desc* desc, void** out_world) {
   w->coop_edge = fit(bb_edge_coloring_blocks(w->sms), w->cap_n, 1024);
   w->coop_pgs = bb_pgs_soft_blocks(w->sms, w->cap_n);
   onesweep_smem_attr();
-  w->coop_avbd = fit(bb_avbd_blocks(w->sms), w->cap_n / 2, 512);
+  w->coop_avbd = bb_avbd_blocks(w->sms, w->cap_n);
+  w->coop_avbd_color = fit(bb_avbd_color_blocks(w->sms), w->cap_n / 2, 512);
   w->coop_cc = fit(bb_components_blocks(w->sms), w->cap_n, 512);
   // The zero fills run on the world's stream ahead of everything the world does later.  On a
   // stream of its own, wait for them here (no device-wide wait); on the caller's stream, which may
@@ -1317,7 +1318,7 @@ bb_status bb_step(void* world, float dt, uint32_t substeps) {
       if (coloured || w->params.solver == BB_SOLVER_AVBD)
         bb_edge_coloring(w->stream, w->d, w->params, w->n, w->sc, w->sms, cur, w->coop_edge);
       cudaEventRecord(ev[10], w->stream);
-      if (w->params.solver == BB_SOLVER_AVBD) bb_solve_avbd(w->stream, w->d, w->params, w->n, h, w->sc, w->sms, cur, w->coop_avbd);
+      if (w->params.solver == BB_SOLVER_AVBD) bb_solve_avbd(w->stream, w->d, w->params, w->n, h, w->sc, w->sms, cur, w->coop_avbd, w->coop_avbd_color);
       else if (!coloured) bb_solve_islands(w->stream, w->d, w->params, w->n, h, cur, w->sc, w->sms);
       else bb_solve_pgs_soft(w->stream, w->d, w->params, w->n, h, cur, w->sc, w->coop_pgs, w->sms);
       cudaEventRecord(ev[11], w->stream);
