@@ -507,7 +507,11 @@ __device__ __forceinline__ void pgs_rows_load(const DevState& d, uint32_t cc, ui
 
 struct PgsItem {
   float3 n, t0, t1, aa, ab;
-  float ima, imb, mu;
+  float ima, imb, mu, cm, ci;  // inverse masses, friction, soft coefficients
+};
+// the two soft-coefficient pairs (solvers.slang:150-158): a contact with a static body, and not
+struct PgsCoef {
+  float m[2], i[2];
 };
 __device__ __forceinline__ PgsItem pgs_item_load(const DevState& d, uint32_t k) {
   const size_t P = d.pair_capacity;
@@ -524,27 +528,33 @@ __device__ __forceinline__ PgsItem pgs_item_load(const DevState& d, uint32_t k) 
   x.ab = make_float3(f3_.w, g.x, g.y);
   return x;
 }
+// (apart from the load: its use of the masses would wait for them before the rows are asked for)
+__device__ __forceinline__ void pgs_item_coef(PgsItem& x, const PgsCoef& co) {
+  const bool fixed = x.ima == 0.f || x.imb == 0.f;
+  x.cm = fixed ? co.m[1] : co.m[0];
+  x.ci = fixed ? co.i[1] : co.i[0];
+}
 
-// the two soft-coefficient pairs (solvers.slang:150-158): a contact with a static body, and not
-struct PgsCoef {
-  float m[2], i[2];
-};
-
-// one contact of an item: warm start (mode 0), solve sweep (1) or relax sweep (2)
-__device__ __forceinline__ void pgs_run_contact(const PgsItem& x, float4 A, float2 B, float4& L, int mode, bool accum,
-                                                bool fric, const PgsCoef& co, const Sym3& IA, const Sym3& IB, float3& va,
-                                                float3& wa, float3& vb, float3& wb) {
+// One contact of an item, in a solve or relax sweep, and in the warm start.  PLAIN: impulses are
+// accumulated and friction is on (the defaults), known at compile time: a contact is one dependent
+// chain of some 40 operations, and each branch on a run-time flag in it costs as much as five of them.
+template <bool PLAIN>
+__device__ __forceinline__ void pgs_run_contact(const PgsItem& x, float4 A, float2 B, float4& L, bool use_bias, uint32_t flags,
+                                                const Sym3& IA, const Sym3& IB, float3& va, float3& wa, float3& vb,
+                                                float3& wb) {
+  const bool accum = PLAIN || (flags & BB_SIM_ACCUM_IMPULSE), fric = PLAIN || (flags & BB_SIM_FRICTION);
   const float3 r1 = xsub(f3(A), x.aa), r2 = xsub(f3(A), x.ab);
-  if (mode == 0) {
-    pgs_contact_warm(r1, r2, L, x.n, x.t0, x.t1, fric, x.ima, x.imb, IA, IB, va, wa, vb, wb);
-  } else {
-    const int q = (x.ima == 0.f || x.imb == 0.f) ? 1 : 0;
-    const float bias = L.w;
-    float4 lam = L;
-    pgs_contact_solve(f4(r1, A.w), f4(r2, B.x), make_float4(B.y, bias, q ? co.m[1] : co.m[0], q ? co.i[1] : co.i[0]), lam,
-                      x.n, x.t0, x.t1, x.mu, mode == 1, accum, fric, x.ima, x.imb, IA, IB, va, wa, vb, wb);
-    L = make_float4(lam.x, lam.y, lam.z, bias);
-  }
+  const float bias = L.w;
+  float4 lam = L;
+  pgs_contact_solve(f4(r1, A.w), f4(r2, B.x), make_float4(B.y, bias, x.cm, x.ci), lam, x.n, x.t0, x.t1, x.mu, use_bias, accum,
+                    fric, x.ima, x.imb, IA, IB, va, wa, vb, wb);
+  L = make_float4(lam.x, lam.y, lam.z, bias);
+}
+template <bool PLAIN>
+__device__ __forceinline__ void pgs_warm_contact(const PgsItem& x, float4 A, float4 L, uint32_t flags, const Sym3& IA,
+                                                 const Sym3& IB, float3& va, float3& wa, float3& vb, float3& wb) {
+  pgs_contact_warm(xsub(f3(A), x.aa), xsub(f3(A), x.ab), L, x.n, x.t0, x.t1, PLAIN || (flags & BB_SIM_FRICTION), x.ima, x.imb,
+                   IA, IB, va, wa, vb, wb);
 }
 
 // gives up a tagged wait past the world's limit, or when another wait already did
@@ -559,12 +569,12 @@ __device__ __forceinline__ bool pgs_gave_up(DevCounters* c, uint32_t spins) {
 }
 
 // sweeps [s0, s1): those below warm are the warm start, those below mid solve, the rest relax
+template <bool PLAIN>
 __device__ __forceinline__ void pgs_sweeps(const DevState& d, const Params& p, const PgsTiles& ft, const PgsCoef& co,
                                            uint32_t s0, uint32_t s1, uint32_t warm, uint32_t mid, bool& dead) {
   const uint32_t T = ft.first[BB_MAX_COLORS];
   const uint32_t w0 = (threadIdx.x >> 5) * gridDim.x + blockIdx.x, nw = gridDim.x * (BB_PGS_THREADS / 32);
   if (w0 >= T || s0 >= s1) return;
-  const bool accum = p.flags & BB_SIM_ACCUM_IMPULSE, fric = p.flags & BB_SIM_FRICTION;
   const bool single = w0 + nw >= T;  // this warp's only tile stays in registers
   float4* vw = pgs_vw(d);
   uint32_t t = w0, s = s0;
@@ -626,16 +636,28 @@ __device__ __forceinline__ void pgs_sweeps(const DevState& d, const Params& p, c
       bodies(!okA, !okB);
       dead = __any_sync(0xFFFFFFFFu, pgs_gave_up(d.ctr, ++spins));
     }
-    const int mode = s < warm ? 0 : s < mid ? 1 : 2;
     float3 va = f3(va4), wa = f3(wa4), vb = f3(vb4), wb = f3(wb4);
-#pragma unroll
-    for (int j = 0; j < BB_PGS_PF; ++j)
-      if (cc > uint32_t(j)) pgs_run_contact(x, r.A[j], r.B[j], r.L[j], mode, accum, fric, co, IA, IB, va, wa, vb, wb);
-    if (deep) {
+    pgs_item_coef(x, co);
+    if (s < warm) {
 #pragma unroll
       for (int j = 0; j < BB_PGS_PF; ++j)
-        if (cc > uint32_t(BB_PGS_PF + j))
-          pgs_run_contact(x, y.A[j], y.B[j], y.L[j], mode, accum, fric, co, IA, IB, va, wa, vb, wb);
+        if (cc > uint32_t(j)) pgs_warm_contact<PLAIN>(x, r.A[j], r.L[j], p.flags, IA, IB, va, wa, vb, wb);
+      if (deep) {
+#pragma unroll
+        for (int j = 0; j < BB_PGS_PF; ++j)
+          if (cc > uint32_t(BB_PGS_PF + j)) pgs_warm_contact<PLAIN>(x, y.A[j], y.L[j], p.flags, IA, IB, va, wa, vb, wb);
+      }
+    } else {
+      const bool use_bias = s < mid;
+#pragma unroll
+      for (int j = 0; j < BB_PGS_PF; ++j)
+        if (cc > uint32_t(j)) pgs_run_contact<PLAIN>(x, r.A[j], r.B[j], r.L[j], use_bias, p.flags, IA, IB, va, wa, vb, wb);
+      if (deep) {
+#pragma unroll
+        for (int j = 0; j < BB_PGS_PF; ++j)
+          if (cc > uint32_t(BB_PGS_PF + j))
+            pgs_run_contact<PLAIN>(x, y.A[j], y.B[j], y.L[j], use_bias, p.flags, IA, IB, va, wa, vb, wb);
+      }
     }
     // the bodies first: other warps wait for them
     if (rec.x >> 31) {
@@ -646,7 +668,7 @@ __device__ __forceinline__ void pgs_sweeps(const DevState& d, const Params& p, c
       st_tagged(vw + 2 * size_t(b), vb, nb + 1u);
       st_tagged(vw + 2 * size_t(b) + 1, wb, nb + 1u);
     }
-    if (mode != 0) {
+    if (s >= warm) {
 #pragma unroll
       for (int j = 0; j < BB_PGS_PF; ++j) {
         if (cc > uint32_t(j)) d.pgs_lam[r.at[j]] = r.L[j];
@@ -666,9 +688,9 @@ __device__ __forceinline__ void pgs_sweeps(const DevState& d, const Params& p, c
 __device__ __forceinline__ void pgs_overflow_item(const DevState& d, const Params& p, uint32_t k, int mode,
                                                   const PgsCoef& co) {
   const uint4 rec = d.pgs_rec[k];
-  const bool accum = p.flags & BB_SIM_ACCUM_IMPULSE, fric = p.flags & BB_SIM_FRICTION;
   const uint32_t a = PGS_BODY(rec.x), b = PGS_BODY(rec.y), cc = rec.z & 15u;
-  const PgsItem x = pgs_item_load(d, k);
+  PgsItem x = pgs_item_load(d, k);
+  pgs_item_coef(x, co);
   const Sym3 IA = load_iw(d, a), IB = load_iw(d, b);
   float4* vw = pgs_vw(d);
   const float4 va4 = ld_tagged(vw + 2 * size_t(a)), wa4 = ld_tagged(vw + 2 * size_t(a) + 1);
@@ -676,7 +698,8 @@ __device__ __forceinline__ void pgs_overflow_item(const DevState& d, const Param
   float3 va = f3(va4), wa = f3(wa4), vb = f3(vb4), wb = f3(wb4);
   for (uint32_t j = rec.w; j < rec.w + cc; ++j) {
     float4 L = d.pgs_lam[j];
-    pgs_run_contact(x, d.c_r1[j], pgs_tmass(d)[j], L, mode, accum, fric, co, IA, IB, va, wa, vb, wb);
+    if (mode == 0) pgs_warm_contact<false>(x, d.c_r1[j], L, p.flags, IA, IB, va, wa, vb, wb);
+    else pgs_run_contact<false>(x, d.c_r1[j], pgs_tmass(d)[j], L, mode == 1, p.flags, IA, IB, va, wa, vb, wb);
     d.pgs_lam[j] = L;
   }
   if (rec.x >> 31) {
@@ -689,6 +712,7 @@ __device__ __forceinline__ void pgs_overflow_item(const DevState& d, const Param
   }
 }
 
+template <bool PLAIN>
 __global__ void __launch_bounds__(BB_PGS_THREADS, BB_PGS_PER_SM) k_pgs_soft(const DevState d, Params p, uint32_t n, float h) {
   __shared__ PgsTiles ft;
   // test switch (bb_debug_wait_limit): the last block leaves, so the others' waits for it run out
@@ -719,7 +743,7 @@ __global__ void __launch_bounds__(BB_PGS_THREADS, BB_PGS_PER_SM) k_pgs_soft(cons
     }
     if (s >= last) break;
     const uint32_t e = o0 != o1 ? s + 1u : s < mid ? mid : last;
-    pgs_sweeps(d, p, ft, co, s, e, warm, mid, dead);
+    pgs_sweeps<PLAIN>(d, p, ft, co, s, e, warm, mid, dead);
     if (o0 != o1) {  // overflow bucket: serial, in manifold order
       grid_sync(d.ctr, sync, epoch);
       if (tid == 0)
@@ -773,7 +797,10 @@ __global__ void k_pgs_finish(const DevState d, Params p, int cur, uint32_t n, fl
 // blocks of k_pgs_soft per SM (one unit of its grid) that are resident together
 static int pgs_blocks_per_sm() {
   int per_sm = 0;
-  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, (const void*)k_pgs_soft, BB_PGS_THREADS, 0);
+  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, (const void*)k_pgs_soft<true>, BB_PGS_THREADS, 0);
+  int other = 0;
+  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&other, (const void*)k_pgs_soft<false>, BB_PGS_THREADS, 0);
+  per_sm = std::min(per_sm, other);
   return std::max(1, std::min(per_sm, BB_PGS_PER_SM));
 }
 
@@ -799,7 +826,9 @@ void bb_solve_pgs_soft(cudaStream_t s, const DevState& d, const Params& p, uint3
   uint32_t nn = n;
   float hh = h;
   void* args[] = {&dd, &pp, &nn, &hh};
-  bb_launch_coop((const void*)k_pgs_soft, coop_blocks, BB_PGS_THREADS, args, s);
+  const uint32_t both = BB_SIM_ACCUM_IMPULSE | BB_SIM_FRICTION;
+  bb_launch_coop((p.flags & both) == both ? (const void*)k_pgs_soft<true> : (const void*)k_pgs_soft<false>, coop_blocks,
+                 BB_PGS_THREADS, args, s);
   k_pgs_finish<<<sms * 8, T, 0, s>>>(d, p, cur, n, h);
 }
 
