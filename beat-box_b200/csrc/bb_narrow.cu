@@ -741,15 +741,14 @@ __global__ void __launch_bounds__(256) k_narrow_carry(const DevState d, int cur,
 
 // Basis, warm start from the previous substep (Manifold::update_from_old,
 // extensions.slang:306-473, after find_old_collision, collision_detection.slang:914-963) and
-// the write of slot k.  Voxel manifolds (vox) inherit only from the old manifold of the same
-// key in the same body order, match features by the whole voxel/corner id, and keep their
-// own depth caps; other manifolds take the pair's old manifold under any key, either order.
-// old_p / old_f are column buffers (stride ST) that receive the old manifold's contacts
-// (position and depth, feature word) once, for the matching loops below.
+// the write of slot k of a voxel pair, by one thread.  Voxel manifolds inherit only from the old
+// manifold of the same key in the same body order, match features by the whole voxel/corner id, and
+// keep their own depth caps.  old_p / old_f are column buffers (stride ST) that receive the old
+// manifold's contacts (position and depth, feature word) once, for the matching loops below.
 template <int ST>
 __device__ __forceinline__ void np_store(const DevState& d, const Params& p, int cur, int warm, uint32_t k,
                                          uint32_t ida, uint32_t idb, uint32_t fa, float3 pa, float3 pb,
-                                         ContactsT<ST>& m, bool vox, float4* old_p, uint32_t* old_f) {
+                                         ContactsT<ST>& m, float4* old_p, uint32_t* old_f) {
   const int prv = cur ^ 1;
   // compute_basis (extensions.slang:262-272)
   float3 n = m.normal, t0;
@@ -758,8 +757,6 @@ __device__ __forceinline__ void np_store(const DevState& d, const Params& p, int
   t0 = t0 * (1.0f / len3(t0));
   float3 t1 = cross3(t0, n);
   const int cc = m.cc;
-  if (!vox)
-    for (int c = 0; c < cc; ++c) m.set_pen(c, fmaxf(m.pen(c), p.penetration_cap));  // extraction cap (:1575-1578)
   // Each new contact records the old contact it inherits from (src, -1: none) and whether the
   // proximity pass gave it (pass2: then the old features, the tangent sign and anchor roles of
   // a swapped pair apply); the inherited fields are read from the old contact when written.
@@ -774,14 +771,7 @@ __device__ __forceinline__ void np_store(const DevState& d, const Params& p, int
   };
   uint32_t pass2 = 0;
   uint32_t ob = 0;
-  bool swapped = false;
-  float sgn = 1.f;
   int32_t err = 0x7FFFFFFF;
-  // Colour reuse: the same manifold (bodies and key) as last substep carries its colour, and
-  // the old manifold is marked as taken over (an old manifold nobody takes over has ended).
-  uint32_t reuse = BB_NONE;
-  const uint32_t sub_tag = d.ctr->substeps;
-  const bool reuse_ok = d.ctr->gc_coloured + 1u == sub_tag;
   if (warm) {
     // find the pair's manifold of the previous substep on the dynamic body's list
     uint32_t x = (fa & BB_BODY_DYNAMIC) ? ida : idb;
@@ -791,38 +781,26 @@ __device__ __forceinline__ void np_store(const DevState& d, const Params& p, int
     for (uint32_t e = s0; e < s1; ++e) {
       if (d.csr_partner[prv][e] != other) continue;
       const uint32_t os = d.csr_slot[prv][e];
-      if (vox && (d.m_keycc[prv][os].x != m.key || d.m_bodies[prv][os].x != ida)) continue;
+      if (d.m_keycc[prv][os].x != m.key || d.m_bodies[prv][os].x != ida) continue;
       old_slot = os;
-      swapped = d.m_bodies[prv][os].x != ida;
       break;
     }
     if (old_slot != BB_NONE) {
       // Manifold::update_from_old (extensions.slang:306-473)
-      int2 okc = d.m_keycc[prv][old_slot];
-      if (reuse_ok && !vox && okc.x == m.key) {
-        reuse = d.gc_slot_color[prv][old_slot];
-        d.gc_survived[old_slot] = sub_tag;
-      }
-      float4 on4 = d.m_normal[prv][old_slot];
-      sgn = swapped ? -1.f : 1.f;
-      bool cross_key = m.key != okc.x || swapped;
-      bool go = !cross_key || dot3(n, f3(on4) * sgn) > 0.7f;
-      if (go) {
-        const int occ = okc.y;
+      {
+        const int occ = d.m_keycc[prv][old_slot].y;
         uint32_t used_old = 0, matched_new = 0;
         ob = old_slot * BB_MAX_CONTACTS;
         for (int j = 0; j < occ; ++j) {
           old_p[j * ST] = d.c_pos[prv][ob + j];
-          if (!cross_key) old_f[j * ST] = __float_as_uint(d.c_anc_a[prv][ob + j].w);
+          old_f[j * ST] = __float_as_uint(d.c_anc_a[prv][ob + j].w);
         }
-        if (!cross_key) {
+        {
           for (int i = 0; i < cc; ++i) {
             for (int j = 0; j < occ; ++j) {
               if (used_old & (1u << j)) continue;
               float4 op = old_p[j * ST];
-              uint32_t ofp = old_f[j * ST];
-              const uint32_t nfp = m.fp(i);
-              bool feat = vox ? ofp == nfp : (fp_in_inc(ofp) == fp_in_inc(nfp) && fp_out_inc(ofp) == fp_out_inc(nfp));
+              const bool feat = old_f[j * ST] == m.fp(i);
               float3 dp = f3(op) - m.pos(i);
               bool close = dot3(dp, dp) < 0.1f * 0.1f;
               if (feat && close) {
@@ -880,13 +858,12 @@ __device__ __forceinline__ void np_store(const DevState& d, const Params& p, int
       const uint32_t oi = ob + uint32_t(j);
       const bool p2 = (pass2 >> c) & 1u;
       const float4 ol = d.c_lam[prv][oi], okt = d.c_kt[prv][oi], oaa = d.c_anc_a[prv][oi];
-      lam = p2 ? make_float4(ol.x, ol.y * sgn, ol.z, ol.w) : ol;
+      lam = ol;
       kt = make_float2(okt.x, okt.y);
       stick = __float_as_uint(okt.z);
       if (stick != 0) {
-        const float3 a0 = f3(oaa), b0 = f3(d.c_anc_b[prv][oi]);
-        aa = (p2 && swapped) ? b0 : a0;
-        ab = (p2 && swapped) ? a0 : b0;
+        aa = f3(oaa);
+        ab = f3(d.c_anc_b[prv][oi]);
       }
       if (p2) fp = __float_as_uint(oaa.w);
       wc = warm_inc(__float_as_uint(okt.w));
@@ -898,58 +875,301 @@ __device__ __forceinline__ void np_store(const DevState& d, const Params& p, int
     d.c_anc_b[cur][cb + c] = f4(ab, 0.f);
   }
   d.hit[k] = 1;
-  d.gc_reuse[k] = reuse;
+  d.gc_reuse[k] = BB_NONE;
 }
 
-// Narrow phase + warm start: one thread per listed pair.  Each thread owns a column of three
-// shared-memory buffers of eight entries: the clip polygon ping-pongs between columns 0 and 1,
-// the contacts end in column 1 with their feature words beside them, and column 0 then takes
-// the old manifold's contacts for the warm-start match (36 KB per 128-thread block).
+// Narrow phase + warm start of box and sphere pairs.  First half, one thread per listed pair:
+// the pair's contacts, into the thread's column of shared memory (the clip polygon ping-pongs
+// between columns 0 and 1, the contacts end in column 1 with their feature words beside them; 36
+// KB per 128-thread block).  Second half, eight lanes per manifold, four manifolds of the warp at a
+// time: the old manifold of the pair is found, its contacts load one per lane, matched against
+// the new ones (Manifold::update_from_old, extensions.slang:306-473, after find_old_collision,
+// collision_detection.slang:914-963), and lane c writes contact c.  A manifold's contacts lie side
+// by side in each array, so eight lanes read or write one line; one thread per manifold made
+// every access of a warp touch 32 lines, ran the matching loops for 8 of 32 lanes, and spent 70 %
+// of the kernel there.  Bound: round trips to memory (the old and the new contacts, 2 GB per
+// substep of a million boxes).  Narrow phase per substep, before -> after: a million boxes 2.72
+// -> 2.29 ms, 1,024 batched worlds 1.35 -> 1.07 ms, 20k mixed pile 188 -> 146 us, 1,000 boxes 114 ->
+// 94 us.  Tried and slower: pairs sorted by separating axis before the clip (2.98 ms).
 #define BB_NARROW_THREADS 128
-__global__ void __launch_bounds__(BB_NARROW_THREADS) k_narrow(const DevState d, Params p, int cur, int warm) {
-  __shared__ float4 s_col[2][BB_MAX_CONTACTS][BB_NARROW_THREADS];
-  __shared__ uint32_t s_feat[2][BB_MAX_CONTACTS][BB_NARROW_THREADS];
+#define BB_NARROW_PER_SM 6  // 80 registers (some spilled): the second half waits on memory
+#define NP_GROUP 8
+static_assert(NP_GROUP == BB_MAX_CONTACTS, "a lane per contact");
+// a touching pair between the halves: normal and contact count | key << 8; position of a and slot;
+// position of b and body a; body b, its old manifold's slot (BB_NONE: none), key, and contact count
+// | swapped << 8
+struct NpPair {
+  float4 n, pa, pb;
+  uint4 old;
+};
+// The pair's manifold of the previous substep, on the dynamic body's list.  In the first half, by
+// the pair's thread: the lookups of a warp's pairs then wait together (three round trips once, not
+// for every four manifolds).
+__device__ __forceinline__ void np_find_old(const DevState& d, int prv, uint32_t ida, uint32_t idb, bool dyn_a, uint4& old) {
+  const uint32_t x = dyn_a ? ida : idb, other = dyn_a ? idb : ida;
+  const uint32_t s0 = d.csr_start[prv][x], s1 = d.csr_start[prv][x + 1];
+  for (uint32_t e = s0; e < s1; ++e) {
+    if (d.csr_partner[prv][e] != other) continue;
+    const uint32_t os = d.csr_slot[prv][e];
+    const int2 kc = d.m_keycc[prv][os];
+    old = make_uint4(old.x, os, uint32_t(kc.x), uint32_t(kc.y) | (d.m_bodies[prv][os].x != ida ? 1u << 8 : 0u));
+    return;
+  }
+}
+
+// The second half for the manifold of thread `col`'s column (col == BB_NONE: this group has none
+// and only takes part in the shuffles; all lanes of the warp call this together).
+__device__ __forceinline__ void np_store_group(const DevState& d, const Params& p, int cur, int warm, uint32_t col,
+                                               const NpPair* pairs, const float4* contacts, const uint32_t* feats) {
   constexpr int ST = BB_NARROW_THREADS;
+  constexpr uint32_t ALL = 0xFFFFFFFFu;
+  const int prv = cur ^ 1, lane = int(threadIdx.x & (NP_GROUP - 1)), shift = int(threadIdx.x & 24u);
+  const bool on = col != BB_NONE;
+  auto group = [&](bool v) { return (__ballot_sync(ALL, v) >> shift) & 0xFFu; };
+  NpPair x = {};
+  if (on) x = pairs[col];
+  float3 n = f3(x.n), t0;
+  const uint32_t kc = __float_as_uint(x.n.w), k = __float_as_uint(x.pa.w), ida = __float_as_uint(x.pb.w), idb = x.old.x;
+  const int cc = int(kc & 0xFFu), key = int(kc >> 8);
+  // compute_basis (extensions.slang:262-272)
+  if (fabsf(n.x) > fabsf(n.y)) t0 = make_float3(n.z, 0.f, -n.x);
+  else t0 = make_float3(0.f, -n.z, n.y);
+  t0 = t0 * (1.0f / len3(t0));
+  float3 t1 = cross3(t0, n);
+  float4 mine = make_float4(0.f, 0.f, 0.f, 0.f);  // this lane's new contact
+  uint32_t fp = 0;
+  if (lane < cc) {
+    mine = contacts[lane * ST + col];
+    mine.w = fmaxf(mine.w, p.penetration_cap);  // extraction cap (:1575-1578)
+    fp = feats[lane * ST + col];
+  }
+  // The old contact this lane's contact inherits from (-1: none), and whether the proximity pass
+  // gave it (then the old features, the tangent sign and anchor roles of a swapped pair apply).
+  int src = -1;
+  bool near = false, swapped = false;
+  float sgn = 1.f;
+  int32_t err = 0x7FFFFFFF;
+  // Colour reuse: the same manifold (bodies and key) as last substep carries its colour, and
+  // the old manifold is marked as taken over (an old manifold nobody takes over has ended).
+  uint32_t reuse = BB_NONE, ob = 0;
+  float4 op = make_float4(0.f, 0.f, 0.f, 0.f), olam = op, okt = op, oaa = op;  // old contact `lane`
+  if (warm) {
+    const uint32_t sub_tag = d.ctr->substeps;
+    const bool reuse_ok = d.ctr->gc_coloured + 1u == sub_tag;
+    const uint32_t old_slot = on ? x.old.y : BB_NONE;
+    int occ = 0;
+    bool go = false, cross_key = false;
+    if (old_slot != BB_NONE) {
+      const int2 okc = make_int2(int(x.old.z), int(x.old.w & 0xFFu));
+      const float4 on4 = d.m_normal[prv][old_slot];
+      swapped = x.old.w >> 8 != 0u;
+      ob = old_slot * BB_MAX_CONTACTS;
+      if (lane < okc.y) {
+        op = d.c_pos[prv][ob + lane];
+        oaa = d.c_anc_a[prv][ob + lane];
+        olam = d.c_lam[prv][ob + lane];
+        okt = d.c_kt[prv][ob + lane];
+      }
+      if (reuse_ok && okc.x == key) {
+        reuse = d.gc_slot_color[prv][old_slot];
+        if (lane == 0) d.gc_survived[old_slot] = sub_tag;
+      }
+      sgn = swapped ? -1.f : 1.f;
+      cross_key = key != okc.x || swapped;
+      go = !cross_key || dot3(n, f3(on4) * sgn) > 0.7f;
+      if (go) occ = okc.y;
+    }
+    const uint32_t ofp = __float_as_uint(oaa.w);
+    uint32_t used = 0, matched = 0;  // old and new contacts taken (the same in all lanes of the group)
+    const int cmax = __reduce_max_sync(ALL, cc);
+    // by features: each new contact takes the first free old one with its features, 10 cm away at most
+    for (int i = 0; i < cmax; ++i) {
+      const float3 pi = make_float3(__shfl_sync(ALL, mine.x, i, NP_GROUP), __shfl_sync(ALL, mine.y, i, NP_GROUP),
+                                    __shfl_sync(ALL, mine.z, i, NP_GROUP));
+      const uint32_t nfp = __shfl_sync(ALL, fp, i, NP_GROUP);
+      const bool feat = fp_in_inc(ofp) == fp_in_inc(nfp) && fp_out_inc(ofp) == fp_out_inc(nfp);
+      const float3 dp = f3(op) - pi;
+      const bool close = dot3(dp, dp) < 0.1f * 0.1f;
+      const uint32_t f = group(!cross_key && i < cc && lane < occ && !(used >> lane & 1u) && feat && close);
+      const int j = f ? __ffs(f) - 1 : 0;
+      const float3 pj = make_float3(__shfl_sync(ALL, op.x, j, NP_GROUP), __shfl_sync(ALL, op.y, j, NP_GROUP),
+                                    __shfl_sync(ALL, op.z, j, NP_GROUP));
+      if (f) {
+        used |= 1u << j;
+        matched |= 1u << i;
+        if (lane == i) {
+          src = j;
+          const float3 d2 = f3(mine) - pj;
+          if (dot3(d2, d2) < 0.01f) mine = f4(pj, mine.w);
+        }
+      }
+    }
+    // by distance: the closest free pair of contacts (35 cm at most), the first in (new, old) order
+    // where two are as close, until none is left
+    for (int round = 0; round < cmax; ++round) {
+      const bool open = go && uint32_t(__popc(matched)) < uint32_t(cc) && uint32_t(__popc(used)) < uint32_t(occ);
+      if (!__any_sync(ALL, open)) break;
+      float best = 0.1225f;
+      int bi = -1, bj = lane;
+      for (int i = 0; i < cmax; ++i) {
+        const float3 pi = make_float3(__shfl_sync(ALL, mine.x, i, NP_GROUP), __shfl_sync(ALL, mine.y, i, NP_GROUP),
+                                      __shfl_sync(ALL, mine.z, i, NP_GROUP));
+        const float3 dp = pi - f3(op);
+        const float d2 = dot3(dp, dp);
+        if (open && i < cc && lane < occ && !(matched >> i & 1u) && !(used >> lane & 1u) && d2 < best) {
+          best = d2;
+          bi = i;
+        }
+      }
+#pragma unroll
+      for (int o = NP_GROUP / 2; o > 0; o >>= 1) {
+        const float b2 = __shfl_xor_sync(ALL, best, o, NP_GROUP);
+        const int i2 = __shfl_xor_sync(ALL, bi, o, NP_GROUP), j2 = __shfl_xor_sync(ALL, bj, o, NP_GROUP);
+        if (i2 >= 0 && (bi < 0 || b2 < best || (b2 == best && (i2 < bi || (i2 == bi && j2 < bj))))) {
+          best = b2;
+          bi = i2;
+          bj = j2;
+        }
+      }
+      if (bi < 0) {
+        go = false;  // (no more rounds for this group; its matches stand)
+      } else {
+        matched |= 1u << bi;
+        used |= 1u << bj;
+        if (lane == bi) {
+          src = bj;
+          near = true;
+        }
+      }
+    }
+    float deep_new = lane < cc ? fminf(0.f, mine.w) : 0.f, deep_old = lane < occ ? fminf(0.f, op.w) : 0.f;
+#pragma unroll
+    for (int o = NP_GROUP / 2; o > 0; o >>= 1) {
+      deep_new = fminf(deep_new, __shfl_xor_sync(ALL, deep_new, o, NP_GROUP));
+      deep_old = fminf(deep_old, __shfl_xor_sync(ALL, deep_old, o, NP_GROUP));
+    }
+    if (occ > 0) err = int32_t(fminf(fmaxf((deep_new - deep_old) * 10000.0f, -32000.0f), 32000.0f));
+  }
+  // the old contact's fields, from its lane
+  const int j = src < 0 ? 0 : src;
+  auto from = [&](float4 v) {
+    return make_float4(__shfl_sync(ALL, v.x, j, NP_GROUP), __shfl_sync(ALL, v.y, j, NP_GROUP), __shfl_sync(ALL, v.z, j, NP_GROUP),
+                       __shfl_sync(ALL, v.w, j, NP_GROUP));
+  };
+  const float4 ol = from(olam), ok = from(okt), oa = from(oaa);
+  if (!on) return;
+  if (lane == 0) {
+    d.m_bodies[cur][k] = make_uint2(ida, idb);
+    d.m_keycc[cur][k] = make_int2(key, cc);
+    d.hit[k] = 1;
+    d.gc_reuse[k] = reuse;
+  } else if (lane == 1) {
+    d.m_normal[cur][k] = f4(n, __int_as_float(err));
+  } else if (lane == 2) {
+    d.m_t0[cur][k] = f4(t0, 0.f);
+  } else if (lane == 3) {
+    d.m_t1[cur][k] = f4(t1, 0.f);
+  } else if (lane == 4) {
+    d.m_anchor_a[cur][k] = make_float4(x.pa.x, x.pa.y, x.pa.z, 0.f);
+  } else if (lane == 5) {
+    d.m_anchor_b[cur][k] = make_float4(x.pb.x, x.pb.y, x.pb.z, 0.f);
+  }
+  if (lane >= cc) return;
+  // new contacts start at zero; matched ones inherit impulses, penalties, stick and anchors
+  float4 lam = make_float4(0.f, 0.f, 0.f, 0.f);
+  float2 kt = make_float2(0.f, 0.f);
+  uint32_t stick = 0, wc = 0;
+  float3 aa = make_float3(0.f, 0.f, 0.f), ab = make_float3(0.f, 0.f, 0.f);
+  if (src >= 0) {
+    lam = near ? make_float4(ol.x, ol.y * sgn, ol.z, ol.w) : ol;
+    kt = make_float2(ok.x, ok.y);
+    stick = __float_as_uint(ok.z);
+    if (stick != 0) {
+      const float3 a0 = f3(oa), b0 = f3(d.c_anc_b[prv][ob + uint32_t(src)]);
+      aa = (near && swapped) ? b0 : a0;
+      ab = (near && swapped) ? a0 : b0;
+    }
+    if (near) fp = __float_as_uint(oa.w);
+    wc = warm_inc(__float_as_uint(ok.w));
+  }
+  const uint32_t ci = k * BB_MAX_CONTACTS + uint32_t(lane);
+  d.c_pos[cur][ci] = mine;
+  d.c_lam[cur][ci] = lam;
+  d.c_kt[cur][ci] = make_float4(kt.x, kt.y, __uint_as_float(stick), __uint_as_float(wc));
+  d.c_anc_a[cur][ci] = f4(aa, __uint_as_float(fp));
+  d.c_anc_b[cur][ci] = f4(ab, 0.f);
+}
+
+__global__ void __launch_bounds__(BB_NARROW_THREADS, BB_NARROW_PER_SM) k_narrow(const DevState d, Params p, int cur, int warm) {
+  __shared__ float4 s_col[2][BB_MAX_CONTACTS][BB_NARROW_THREADS];
+  __shared__ uint32_t s_feat[BB_MAX_CONTACTS][BB_NARROW_THREADS];
+  __shared__ uint8_t s_order[BB_NARROW_THREADS];  // columns of each warp's touching pairs
+  constexpr int ST = BB_NARROW_THREADS;
+  // column 0 is free between the halves: the pairs that touch
+  NpPair* const s_pair = reinterpret_cast<NpPair*>(&s_col[0][0][0]);
+  static_assert(sizeof(NpPair) <= BB_MAX_CONTACTS * sizeof(float4), "a pair fits a thread's column");
   float4* const buf = &s_col[0][0][threadIdx.x];
   const uint32_t S = slot_total(d);
   const uint32_t nbb = d.ctr->np_counts[0], ntot = nbb + d.ctr->np_counts[1];
-  for (uint32_t t = blockIdx.x * blockDim.x + threadIdx.x; t < ntot; t += gridDim.x * blockDim.x) {
-    const uint32_t k = d.np_list[t < nbb ? t : S - 1 - (t - nbb)];
-    uint2 pr = d.pairs[slot_pair_of(d, k)];
-    uint32_t ida = d.vals[0][pr.x], idb = d.vals[0][pr.y];
-    const uint32_t fa = d.flags[ida];
-    float4 pa4 = d.pos[ida], pb4 = d.pos[idb];
-    float4 sa = d.shape[ida], sb = d.shape[idb];
-    Quatf qa = q_from(d.rot[ida]), qb = q_from(d.rot[idb]);
-    float3 pa = f3(pa4), pb = f3(pb4);
-    uint32_t ta = __float_as_uint(sa.w), tb = __float_as_uint(sb.w);
-    ContactsT<ST> m;
-    m.p = &s_col[1][0][threadIdx.x];
-    m.f = &s_feat[1][0][threadIdx.x];
-    bool hit;
-    if (ta == BB_SHAPE_BOX && tb == BB_SHAPE_BOX) {
-      hit = box_box<ST>(qa, pa, f3(sa), qb, pb, f3(sb), (p.quirks & BB_QUIRK_SAT_FRAME) != 0, buf, m);
-    } else if (ta == BB_SHAPE_SPHERE && tb == BB_SHAPE_SPHERE) {
-      hit = sphere_sphere<ST>(pa, sa.x, pb, sb.x, m);
-    } else {
-      float3 n, pos;
-      float pen;
-      if (ta == BB_SHAPE_BOX) {
-        hit = box_sphere_core(qa, pa, f3(sa), pb, sb.x, n, pen, pos);
-        m.key = BB_KEY_BOX_SPHERE;
+  const uint32_t warp0 = threadIdx.x & ~31u;
+  for (uint32_t base = blockIdx.x * blockDim.x; base < ntot; base += gridDim.x * blockDim.x) {  // block-uniform
+    const uint32_t t = base + threadIdx.x;
+    NpPair x = {};
+    bool hit = false;
+    if (t < ntot) {
+      const uint32_t k = d.np_list[t < nbb ? t : S - 1 - (t - nbb)];
+      uint2 pr = d.pairs[slot_pair_of(d, k)];
+      uint32_t ida = d.vals[0][pr.x], idb = d.vals[0][pr.y];
+      const uint32_t fa = d.flags[ida];
+      float4 pa4 = d.pos[ida], pb4 = d.pos[idb];
+      float4 sa = d.shape[ida], sb = d.shape[idb];
+      Quatf qa = q_from(d.rot[ida]), qb = q_from(d.rot[idb]);
+      float3 pa = f3(pa4), pb = f3(pb4);
+      uint32_t ta = __float_as_uint(sa.w), tb = __float_as_uint(sb.w);
+      ContactsT<ST> m;
+      m.p = &s_col[1][0][threadIdx.x];
+      m.f = &s_feat[0][threadIdx.x];
+      if (ta == BB_SHAPE_BOX && tb == BB_SHAPE_BOX) {
+        hit = box_box<ST>(qa, pa, f3(sa), qb, pb, f3(sb), (p.quirks & BB_QUIRK_SAT_FRAME) != 0, buf, m);
+      } else if (ta == BB_SHAPE_SPHERE && tb == BB_SHAPE_SPHERE) {
+        hit = sphere_sphere<ST>(pa, sa.x, pb, sb.x, m);
       } else {
-        hit = box_sphere_core(qb, pb, f3(sb), pa, sa.x, n, pen, pos);
-        n = -n;
-        m.key = BB_KEY_SPHERE_BOX;
+        float3 n, pos;
+        float pen;
+        if (ta == BB_SHAPE_BOX) {
+          hit = box_sphere_core(qa, pa, f3(sa), pb, sb.x, n, pen, pos);
+          m.key = BB_KEY_BOX_SPHERE;
+        } else {
+          hit = box_sphere_core(qb, pb, f3(sb), pa, sa.x, n, pen, pos);
+          n = -n;
+          m.key = BB_KEY_SPHERE_BOX;
+        }
+        if (hit) {
+          m.cc = 1;
+          m.normal = n;
+          m.set(0, pos, pen, fp_pack(m.key, m.key, m.key, m.key));
+        }
       }
       if (hit) {
-        m.cc = 1;
-        m.normal = n;
-        m.set(0, pos, pen, fp_pack(m.key, m.key, m.key, m.key));
+        x = NpPair{f4(m.normal, __uint_as_float(uint32_t(m.cc) | uint32_t(m.key) << 8)), f4(pa, __uint_as_float(k)),
+                   f4(pb, __uint_as_float(ida)), make_uint4(idb, BB_NONE, 0u, 0u)};
+        if (warm) np_find_old(d, cur ^ 1, ida, idb, fa & BB_BODY_DYNAMIC, x.old);
       }
     }
-    if (!hit) continue;
-    np_store<ST>(d, p, cur, warm, k, ida, idb, fa, pa, pb, m, false, buf, &s_feat[0][0][threadIdx.x]);
+    __syncthreads();  // every thread's clip is done with its column
+    const uint32_t hits = __ballot_sync(0xFFFFFFFFu, hit);
+    if (hit) {
+      s_pair[threadIdx.x] = x;
+      s_order[warp0 + uint32_t(__popc(hits & ((1u << (threadIdx.x & 31u)) - 1u)))] = uint8_t(threadIdx.x);
+    }
+    __syncwarp();
+    for (int r = 0; r < __popc(hits); r += 32 / NP_GROUP) {
+      // the (r + group)th touching pair of the warp
+      const int q = r + int((threadIdx.x & 31u) / NP_GROUP);
+      np_store_group(d, p, cur, warm, q < __popc(hits) ? s_order[warp0 + uint32_t(q)] : BB_NONE, s_pair, &s_col[1][0][0],
+                     &s_feat[0][0]);
+    }
+    __syncthreads();  // before the next pairs' clips
   }
 }
 
@@ -1338,7 +1558,7 @@ __global__ void __launch_bounds__(256) k_voxel_narrow(const DevState d, Params p
         m.cc = n_emit;
         store = n_emit > 0;
       }
-      if (store) np_store<1>(d, p, cur, warm, slot0 + code, ida, idb, d.flags[ida], A.p, B.p, m, true, lo, lof);
+      if (store) np_store<1>(d, p, cur, warm, slot0 + code, ida, idb, d.flags[ida], A.p, B.p, m, lo, lof);
     }
     __syncwarp();
   }
