@@ -5,7 +5,7 @@
 // src/shaders/simulation/LBVH.slang:34-152, RBM:1288-1295) with:
 //   * one histogram kernel that counts all digit positions in a single read of the keys,
 //   * one onesweep kernel per digit: tiles of 8192 keys rank themselves with warp-level
-//     multisplit (one ballot per digit bit), publish per-digit tile totals, resolve their global
+//     multisplit (the lanes of a digit found through mask words in shared memory), publish per-digit tile totals, resolve their global
 //     offsets by decoupled look-back over the preceding tiles, reorder the tile by digit in
 //     shared memory and write each digit's run contiguously (coalesced stores).
 // Both are stable, so the result equals a stable sort by key -- the reference's semantics.
@@ -223,9 +223,15 @@ __device__ __forceinline__ uint32_t sort_lookback(volatile uint32_t* st, uint32_
 // each), so each digit's run in a tile averages 32 keys (128-byte lines when written out).  The
 // values are read when the tile is reordered, not held through the ranking (registers: two
 // blocks per SM); with a lut the digit needs the value, which the ranking reads then.
+// Bound: instruction issue and shared memory in the ranking, then the look-back.  With a ballot per
+// digit bit (8 ballots and selects per key) the ranking took half of the issue slots: 2^24 random
+// pairs 644 -> 545 us, constant keys 611 -> 468 us, 10,000 pairs 69 -> 60 us.  Longer look-back
+// loads (16 or 32 words) were slower (660, 688 us before the change).
 // Shared memory (dynamic, kSortSmem bytes): per-warp digit counts 16 x 256, keys and values of
 // the tile, the digit of each reordered position.
 constexpr int kSortWarps = kSortThreads / 32;
+constexpr int kSortMasks = 4;  // keys of a thread ranked together (2 measured the same)
+static_assert(kSortWarps * kSortMasks * 256 <= 2 * BB_SORT_TILE && kSortItems % kSortMasks == 0, "mask words");
 constexpr size_t kSortSmem = size_t(kSortWarps) * 256 * 4 + size_t(BB_SORT_TILE) * (4 + 4 + 1);
 __global__ void __launch_bounds__(kSortThreads, 2) k_onesweep(const uint32_t* __restrict__ keys_in,
                                                               const uint32_t* __restrict__ vals_in,
@@ -260,30 +266,48 @@ __global__ void __launch_bounds__(kSortThreads, 2) k_onesweep(const uint32_t* __
     const uint32_t i = first + k * 32;
     key[k] = i < n ? keys_in[i] : 0u;
   }
-  // warp-level multisplit: rank of each key among its warp's keys of the same digit, in order.
-  // The lanes holding the same digit are found with one ballot per digit bit (plus one for the
-  // keys past n); only the lowest of them reads and advances the warp's count of that digit, and
-  // the others take the old count from it by a shuffle.  rank keeps the digit in its top 8 bits.
+  // Warp-level multisplit: rank of each key among its warp's keys of the same digit, in order.
+  // Every lane sets its bit in its digit's mask word; the word then names the lanes with that
+  // digit, and the lowest of them advances the warp's count of the digit and hands the old count to
+  // the others by a shuffle.  kSortMasks keys of a thread are in flight, each with mask words of its own
+  // (they lie where the reordered keys and values go later).  rank keeps the digit in its top 8 bits.
+  uint32_t* masks = s_keys + warp * (kSortMasks * 256);
 #pragma unroll
-  for (int k = 0; k < kSortItems; ++k) {
-    const bool valid = first + k * 32 < n;
-    const uint32_t d = valid ? sort_digit(key[k], lut ? vals_in[first + k * 32] : 0u, lut, shift) : 0u;
-    uint32_t peers = __ballot_sync(0xFFFFFFFFu, valid);
-    if (!valid) peers = ~peers;
+  for (int i = 0; i < kSortMasks * 256 / 32; ++i) masks[i * 32 + lane] = 0u;
+  __syncwarp();
 #pragma unroll
-    for (int b = 0; b < 8; ++b) {
-      const uint32_t bal = __ballot_sync(0xFFFFFFFFu, (d >> b) & 1u);
-      peers &= ((d >> b) & 1u) ? bal : ~bal;
+  for (int k0 = 0; k0 < kSortItems; k0 += kSortMasks) {
+    uint32_t dig[kSortMasks], peers[kSortMasks], prior[kSortMasks];
+#pragma unroll
+    for (int j = 0; j < kSortMasks; ++j) {
+      const uint32_t i = first + (k0 + j) * 32;
+      dig[j] = i < n ? sort_digit(key[k0 + j], lut ? vals_in[i] : 0u, lut, shift) : 256u;
+      // one digit in the whole warp (high digits of nearly sorted keys): no mask, whose 32
+      // additions to one word would run one after the other
+      int same;
+      __match_all_sync(0xFFFFFFFFu, dig[j], &same);
+      peers[j] = same ? 0xFFFFFFFFu : 0u;
+      if (!same && dig[j] < 256u) atomicOr(&masks[j * 256 + dig[j]], 1u << lane);
     }
-    const int leader = __ffs(peers) - 1;
-    uint32_t prior = 0;
-    if (valid && lane == leader) {
-      prior = s_warp_hist[warp][d];
-      s_warp_hist[warp][d] = prior + __popc(peers);
-    }
-    prior = __shfl_sync(0xFFFFFFFFu, prior, leader);
-    rank[k] = (d << 24) | (prior + __popc(peers & lt_mask));
     __syncwarp();
+#pragma unroll
+    for (int j = 0; j < kSortMasks; ++j)
+      if (peers[j] == 0u) peers[j] = dig[j] < 256u ? masks[j * 256 + dig[j]] : 1u << lane;
+    __syncwarp();
+#pragma unroll
+    for (int j = 0; j < kSortMasks; ++j) {
+      prior[j] = 0u;
+      if (dig[j] < 256u && (peers[j] & lt_mask) == 0u) {
+        prior[j] = atomicAdd(&s_warp_hist[warp][dig[j]], uint32_t(__popc(peers[j])));
+        masks[j * 256 + dig[j]] = 0u;
+      }
+      __syncwarp();  // the next key's leader of the same digit counts on
+    }
+#pragma unroll
+    for (int j = 0; j < kSortMasks; ++j) {
+      const uint32_t p = __shfl_sync(0xFFFFFFFFu, prior[j], __ffs(peers[j]) - 1);
+      rank[k0 + j] = (dig[j] << 24) | (p + __popc(peers[j] & lt_mask));
+    }
   }
   __syncthreads();
   // per digit t (threads 0..255): exclusive prefix over warps, and the tile's count of digit t
