@@ -1085,6 +1085,39 @@ __global__ void __launch_bounds__(BB_COOP_THREADS, 1) k_avbd_color(const DevStat
   for (uint32_t i = tid; i < n; i += stride) {
     uint32_t v = d.body_color[i];
     d.body_color[i] = v == BB_UNCOLORED ? BB_UNCOLORED : (v & 255u);
+    d.a_depth[i] = awake(d.flags[i]) ? BB_NONE : 0u;
+  }
+  // Support depth (avbd.slang:667-724): breadth-first from the bodies at rest, one pass over the
+  // manifolds per shock layer, until a pass lowers no depth (the reference dispatches all passes;
+  // the later ones change nothing).
+  grid_sync(c, sync, ep);  // the colouring's last flags are read
+  if (tid == 0) {
+    uncol[0] = 0;
+    uncol[1] = 0;
+  }
+  grid_sync(c, sync, ep);
+  const uint32_t M = c->manifold_count;
+  for (uint32_t k = 0; k < p.avbd_shock_layers; ++k) {
+    bool lower = false;
+    for (uint32_t m = tid; m < M; m += stride) {
+      const uint32_t slot = d.man_slot[cur][m];
+      if (d.m_keycc[cur][slot].y <= 0) continue;
+      const uint2 b = d.m_bodies[cur][slot];
+      const uint32_t d1 = *(volatile uint32_t*)&d.a_depth[b.x], d2 = *(volatile uint32_t*)&d.a_depth[b.y];
+      if (d2 != BB_NONE && d2 + 1u < d1) {
+        atomicMin(&d.a_depth[b.x], d2 + 1u);
+        lower = true;
+      }
+      if (d1 != BB_NONE && d1 + 1u < d2) {
+        atomicMin(&d.a_depth[b.y], d1 + 1u);
+        lower = true;
+      }
+    }
+    if (lower) atomicOr(&uncol[k & 1], 1u);
+    grid_sync(c, sync, ep);
+    if (*(volatile uint32_t*)&uncol[k & 1] == 0u) break;
+    if (tid == 0) uncol[(k + 1) & 1] = 0;
+    grid_sync(c, sync, ep);
   }
 }
 
@@ -1189,23 +1222,6 @@ __global__ void k_avbd_warmstart(const DevState d, Params p, int cur) {
   }
 }
 
-__global__ void k_avbd_depth_reset(const DevState d, uint32_t n) {
-  uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  d.a_depth[i] = awake(d.flags[i]) ? BB_NONE : 0u;
-}
-__global__ void k_avbd_depth_relax(const DevState d, int cur) {
-  const uint32_t M = d.ctr->manifold_count;
-  for (uint32_t m = blockIdx.x * blockDim.x + threadIdx.x; m < M; m += gridDim.x * blockDim.x) {
-    const uint32_t slot = d.man_slot[cur][m];
-    if (d.m_keycc[cur][slot].y <= 0) continue;
-    const uint2 b = d.m_bodies[cur][slot];
-    uint32_t d1 = *(volatile uint32_t*)&d.a_depth[b.x], d2 = *(volatile uint32_t*)&d.a_depth[b.y];
-    if (d2 != BB_NONE && d2 + 1u < d1) atomicMin(&d.a_depth[b.x], d2 + 1u);
-    if (d1 != BB_NONE && d1 + 1u < d2) atomicMin(&d.a_depth[b.y], d1 + 1u);
-  }
-}
-
 // starts[v] = first sorted position with key >= v * scale, for v in [0, nb]
 __global__ void k_lower_bounds(const uint32_t* keys, uint32_t n, uint32_t* starts, uint32_t nb, uint32_t scale) {
   uint32_t v = blockIdx.x * blockDim.x + threadIdx.x;
@@ -1296,8 +1312,8 @@ __global__ void k_avbd_keys(const DevState d, Params p, uint32_t n, int post) {
     }
     key = key * AVBD_CLASSES + avbd_class(d)[i];
   }
-  d.a_bucket_keys[0][i] = key;
-  d.a_bucket_vals[0][i] = i;
+  (post ? d.bucket_keys[0] : d.a_bucket_keys[0])[i] = key;
+  (post ? d.bucket_vals[0] : d.a_bucket_vals[0])[i] = i;
 }
 // entry_avbd_primal (avbd.slang:478-658): Gauss-Newton step of body i on its 6 DoF, in two
 // parts: the sums over its contacts (avbd_gather) and the solve (avbd_move).
@@ -1565,9 +1581,8 @@ __device__ void avbd_finalize(const DevState& d, int cur, uint32_t i, float dt) 
 // trip.  All lanes sum the contacts; then the block's first lanes solve one body each, so that
 // the 6x6 solve (hundreds of instructions) is issued once per block and trip and not by every warp
 // for its few bodies.  buf alternates, so a trip's sums are written while the last one's are solved.
-__device__ __forceinline__ void avbd_bucket(const DevState& d, const Params& p, int cur, uint32_t s0, uint32_t s1, float dt,
-                                            float alpha, float* sums, uint32_t& trip) {
-  const uint32_t* list = d.a_bucket_vals[1];
+__device__ __forceinline__ void avbd_bucket(const DevState& d, const Params& p, int cur, const uint32_t* list, uint32_t s0,
+                                            uint32_t s1, float dt, float alpha, float* sums, uint32_t& trip) {
   for (uint32_t base = s0 + blockIdx.x * AVBD_BODIES; base < s1; base += gridDim.x * AVBD_BODIES, ++trip) {
     float* buf = sums + (trip & 1u) * 27 * AVBD_BODIES;
     const uint32_t k = base + threadIdx.x / AVBD_LANES;
@@ -1589,18 +1604,20 @@ __global__ void __launch_bounds__(AVBD_THREADS, 512 / AVBD_THREADS) k_avbd_solve
   uint32_t* sync = &d.ctr->sync_count[3 + phase];
   uint32_t ep = 0, trip = 0;
   const uint32_t keys = phase == 1 ? p.avbd_shock_layers * BB_MAX_COLORS : min(d.ctr->avbd_colors, uint32_t(BB_MAX_COLORS));
+  const uint32_t* list = phase == 1 ? d.bucket_vals[0] : d.a_bucket_vals[1];
+  const uint32_t* starts = phase == 1 ? d.a_bucket_start : d.bucket_start;
   if (threadIdx.x < 32u) {
     uint32_t c = 0;
     for (uint32_t k0 = 0; k0 < keys; k0 += 32u) {
       const uint32_t k = k0 + threadIdx.x;
-      const uint32_t a = k < keys ? d.a_bucket_start[k] : 0u;
-      const bool full = k < keys && d.a_bucket_start[k + 1] != a;
+      const uint32_t a = k < keys ? starts[k] : 0u;
+      const bool full = k < keys && starts[k + 1] != a;
       const uint32_t m = __ballot_sync(0xFFFFFFFFu, full);
       if (full) bs[c + uint32_t(__popc(m & ((1u << threadIdx.x) - 1u)))] = a;
       c += uint32_t(__popc(m));
     }
     if (threadIdx.x == 0) {
-      bs[c] = keys ? d.a_bucket_start[keys] : 0u;
+      bs[c] = keys ? starts[keys] : 0u;
       s_nb = c;
     }
   }
@@ -1612,7 +1629,7 @@ __global__ void __launch_bounds__(AVBD_THREADS, 512 / AVBD_THREADS) k_avbd_solve
   const uint32_t M = d.ctr->manifold_count;
   for (uint32_t sw = 0; sw < sweeps; ++sw) {
     for (uint32_t b = 0; b < nb; ++b) {
-      avbd_bucket(d, p, cur, bs[b], bs[b + 1], dt, alpha, sums, trip);
+      avbd_bucket(d, p, cur, list, bs[b], bs[b + 1], dt, alpha, sums, trip);
       grid_sync(d.ctr, sync, ep);
     }
     if (phase == 0) {
@@ -1626,22 +1643,25 @@ __global__ void __launch_bounds__(AVBD_THREADS, 512 / AVBD_THREADS) k_avbd_solve
       if (awake(d.flags[i])) avbd_finalize(d, cur, i, dt);
 }
 
-// Scratch of the body bucket sorts (every region is zeroed once per substep and used once):
-// histogram region `region` (2048 words each), status / tile-counter slots from `slot`.
-static void avbd_buckets(cudaStream_t s, const DevState& d, const Params& p, uint32_t n, const StepScratch& sc,
-                         int sms, int post, int region, int slot) {
+// The body lists of the colour sweeps (post = 0: a_bucket_vals[1], starts in bucket_start) and of the
+// sweep over the support layers (post = 1: bucket_vals[0], starts in a_bucket_start).  Both stay
+// until the solve ends: the last sweeps walk the colour lists again.  bucket_* are the edge
+// colouring's arrays, which AVBD does not read after it.  Scratch: histogram region 2 or 3, status
+// and tile-counter slots 7 or 8 and 9 (every one is zeroed once per substep and used once).
+static void avbd_buckets(cudaStream_t s, const DevState& d, const Params& p, uint32_t n, const StepScratch& sc, int sms,
+                         int post) {
   const int T = BB_THREADS;
   uint32_t blocks = (n + T - 1) / T;
   k_avbd_keys<<<blocks, T, 0, s>>>(d, p, n, post);
-  uint32_t* keys[2] = {d.a_bucket_keys[0], d.a_bucket_keys[1]};
-  uint32_t* vals[2] = {d.a_bucket_vals[0], d.a_bucket_vals[1]};
-  uint32_t* hist = sc.sort_hist + size_t(region) * BB_HIST_REGION;
-  // post keys need up to 14 bits; three 8-bit passes (the third sees only zero digits, so it keeps
-  // the order) leave the result in buffer 1 like the one-pass colour sort
-  bb_launch_sort(s, keys, vals, nullptr, n, post ? 3 : 1, 0, hist, sc.sort_status + size_t(slot) * sc.sort_tiles * 256,
-                 sc.sort_tile_ctr + slot, d.ctr, sms);
-  uint32_t nb = post ? p.avbd_shock_layers * BB_MAX_COLORS : BB_MAX_COLORS;
-  k_lower_bounds<<<(nb + 1 + 127) / 128, 128, 0, s>>>(d.a_bucket_keys[1], n, d.a_bucket_start, nb, AVBD_CLASSES);
+  uint32_t* keys[2] = {post ? d.bucket_keys[0] : d.a_bucket_keys[0], post ? d.bucket_keys[1] : d.a_bucket_keys[1]};
+  uint32_t* vals[2] = {post ? d.bucket_vals[0] : d.a_bucket_vals[0], post ? d.bucket_vals[1] : d.a_bucket_vals[1]};
+  const int slot = post ? 8 : 7;
+  // colour keys fit one 8-bit digit (result in buffer 1), layer keys two (buffer 0)
+  bb_launch_sort(s, keys, vals, nullptr, n, post ? 2 : 1, 0, sc.sort_hist + size_t(post ? 3 : 2) * BB_HIST_REGION,
+                 sc.sort_status + size_t(slot) * sc.sort_tiles * 256, sc.sort_tile_ctr + slot, d.ctr, sms);
+  const uint32_t nb = post ? p.avbd_shock_layers * BB_MAX_COLORS : BB_MAX_COLORS;
+  k_lower_bounds<<<(nb + 1 + 127) / 128, 128, 0, s>>>(keys[post ? 0 : 1], n, post ? d.a_bucket_start : d.bucket_start, nb,
+                                                      AVBD_CLASSES);
 }
 
 int bb_avbd_color_blocks(int sms) { return bb_coop_blocks((const void*)k_avbd_color, BB_COOP_THREADS, sms); }
@@ -1671,8 +1691,6 @@ void bb_solve_avbd(cudaStream_t s, const DevState& d, const Params& p, uint32_t 
   k_avbd_prepare<<<blocks, T, 0, s>>>(d, p, n, h);
   k_avbd_warmstart<<<sms * 8, T, 0, s>>>(d, p, cur);
   k_avbd_entries<<<blocks, T, 0, s>>>(d, n, cur);
-  k_avbd_depth_reset<<<blocks, T, 0, s>>>(d, n);
-  for (uint32_t k = 0; k < p.avbd_shock_layers; ++k) k_avbd_depth_relax<<<sms * 8, T, 0, s>>>(d, cur);
   DevState dd = d;
   Params pp = p;
   int cc = cur;
@@ -1680,14 +1698,13 @@ void bb_solve_avbd(cudaStream_t s, const DevState& d, const Params& p, uint32_t 
   float hh = h;
   int phase = 0;
   void* args[] = {&dd, &pp, &cc, &nn, &hh, &phase};
-  avbd_buckets(s, d, p, n, sc, sms, 0, 2, 7);
+  avbd_buckets(s, d, p, n, sc, sms, 0);
   bb_launch_coop((const void*)k_avbd_solve, coop_blocks, AVBD_THREADS, args, s);
-  avbd_buckets(s, d, p, n, sc, sms, 1, 3, 8);  // slots 8, 9, 10
+  avbd_buckets(s, d, p, n, sc, sms, 1);
   int phase1 = 1;
   void* args1[] = {&dd, &pp, &cc, &nn, &hh, &phase1};
   bb_launch_coop((const void*)k_avbd_solve, coop_blocks, AVBD_THREADS, args1, s);
   if (p.avbd_post_stab_sweeps > 1) {
-    avbd_buckets(s, d, p, n, sc, sms, 0, 4, 11);
     int phase2 = 2;
     void* args2[] = {&dd, &pp, &cc, &nn, &hh, &phase2};
     bb_launch_coop((const void*)k_avbd_solve, coop_blocks, AVBD_THREADS, args2, s);
