@@ -166,7 +166,7 @@ struct DevState {
   uint32_t* gc_color;    // per compact manifold
   uint32_t* gc_pid;      // pair-identity hash
   uint32_t* gc_choice;
-  uint4* gc_rec;         // per compact manifold: body a, body b, pair hash, static bits
+  uint4* gc_rec;         // per compact manifold: body a, body b, pair hash, bits 0..2 static / idle, class << 3
   uint32_t* gc_list[2];  // manifolds still uncoloured after a round (alternating)
   uint32_t* gc_mask;     // per body
   uint32_t* gc_island_tag; // per island: colouring epoch + 1 when one of its bodies is awake

@@ -256,15 +256,38 @@ __device__ __forceinline__ uint32_t gc_priority(uint32_t pid, uint32_t round) {
 //   commit: a manifold that won on both bodies takes the colour (:179-212).
 // Finally writes the (colour, manifold) keys of the bucket sort.
 // Persistent colouring kernel.  Each manifold's bodies, static bits and pair hash are packed
-// into one record up front, so a round touches rec -> body masks -> owner words only; the
+// into one record up front (with the contact-count class for the keys), so a round touches rec -> body masks -> owner words only; the
 // grid barrier is the arrival-counter kind (counter 0 of the substep).
 #define BB_GC_THREADS 1024
-#define GC_UNROLL 3  // list entries a thread takes per trip of a round
+#define GC_UNROLL 3  // entries a thread takes per trip (1M boxes: 1293 / 1138 / 1114 us at 2 / 3 / 4; 4 spills, small worlds lose 4 %)
 // Owner word of (body, colour), colour-major: a round's bids go mostly to the lowest free colours,
 // so the words in use (8 bytes per body for each colour bid) stay in L2, where a body-major
 // table (256 bytes per body) spread every round's random atomics over the whole table in DRAM.
 __device__ __forceinline__ size_t gc_owner_at(const DevState& d, uint32_t body, uint32_t col) {
   return size_t(col) * (size_t(d.body_capacity) + 1u) + body;
+}
+// Appends a warp's taken entries (item of lane and u: m[u]) to a list: one atomic per warp and
+// trip.  All warps add to the same word, so an append per 32 entries queued up there: with this, and
+// GC_UNROLL entries' loads in flight in the first and last passes too, the colouring of 1M boxes
+// (3 M manifolds) fell 1535 -> 1138 us, of 1,024 worlds 433 -> 360 us.
+__device__ __forceinline__ void gc_append(uint32_t* count, uint32_t* list, const bool (&take)[GC_UNROLL],
+                                          const uint32_t (&m)[GC_UNROLL]) {
+  const uint32_t lane = threadIdx.x & 31u, lt = (1u << lane) - 1u;
+  uint32_t mask[GC_UNROLL], total = 0;
+#pragma unroll
+  for (int u = 0; u < GC_UNROLL; ++u) {
+    mask[u] = __ballot_sync(0xFFFFFFFFu, take[u]);
+    total += uint32_t(__popc(mask[u]));
+  }
+  if (total == 0u) return;
+  uint32_t off = 0;
+  if (lane == 0) off = atomicAdd(count, total);
+  off = __shfl_sync(0xFFFFFFFFu, off, 0);
+#pragma unroll
+  for (int u = 0; u < GC_UNROLL; ++u) {
+    if (take[u]) list[off + uint32_t(__popc(mask[u] & lt))] = m[u];
+    off += uint32_t(__popc(mask[u]));
+  }
 }
 __global__ void __launch_bounds__(BB_GC_THREADS, 1) k_edge_color(const DevState d, Params p, int cur, uint32_t n) {
   DevCounters* c = d.ctr;
@@ -317,42 +340,56 @@ __global__ void __launch_bounds__(BB_GC_THREADS, 1) k_edge_color(const DevState 
   grid_sync(c, sync, ep);
   // round 1's list: the manifolds of islands with an awake body (a warp appends its lanes at once)
   uint32_t used0 = 0;  // colour + 1 of the reused colours
-  for (uint32_t base = warp0; base < M; base += stride) {  // warp-uniform trips
-    const uint32_t m = base + lane;
-    bool colour = false;
-    if (m < M) {
-      const uint32_t slot = d.man_slot[cur][m];
-      uint2 b = d.m_bodies[cur][slot];
-      int key = d.m_keycc[cur][slot].x;
-      const uint32_t fa = d.flags[b.x], fb = d.flags[b.y];
-      const bool da = fa & BB_BODY_DYNAMIC, db = fb & BB_BODY_DYNAMIC;
-      const uint32_t isl = da ? d.island[b.x] : db ? d.island[b.y] : BB_NONE;
-      colour = isl != BB_NONE && d.gc_island_tag[isl] == itag;
+  for (uint32_t base = warp0; base < M; base += GC_UNROLL * stride) {  // warp-uniform trips
+    uint32_t slot[GC_UNROLL], fa[GC_UNROLL], fb[GC_UNROLL], isl[GC_UNROLL];
+    uint2 b[GC_UNROLL];
+    int2 kc[GC_UNROLL];
+    bool colour[GC_UNROLL];
+#pragma unroll
+    for (int u = 0; u < GC_UNROLL; ++u) {
+      const uint32_t m = base + uint32_t(u) * stride + lane;
+      slot[u] = m < M ? d.man_slot[cur][m] : BB_NONE;
+    }
+#pragma unroll
+    for (int u = 0; u < GC_UNROLL; ++u) {
+      b[u] = slot[u] != BB_NONE ? d.m_bodies[cur][slot[u]] : make_uint2(0, 0);
+      kc[u] = slot[u] != BB_NONE ? d.m_keycc[cur][slot[u]] : make_int2(0, 0);
+    }
+#pragma unroll
+    for (int u = 0; u < GC_UNROLL; ++u) {
+      fa[u] = slot[u] != BB_NONE ? d.flags[b[u].x] : 0u;
+      fb[u] = slot[u] != BB_NONE ? d.flags[b[u].y] : 0u;
+    }
+#pragma unroll
+    for (int u = 0; u < GC_UNROLL; ++u)
+      isl[u] = (fa[u] & BB_BODY_DYNAMIC) ? d.island[b[u].x] : (fb[u] & BB_BODY_DYNAMIC) ? d.island[b[u].y] : BB_NONE;
+#pragma unroll
+    for (int u = 0; u < GC_UNROLL; ++u) {
+      const uint32_t m = base + uint32_t(u) * stride + lane;
+      colour[u] = isl[u] != BB_NONE && d.gc_island_tag[isl[u]] == itag;
       uint32_t kept = BB_NONE;  // a reused colour
-      if (colour && reuse && d.gc_island_chg[isl] != itag) {
-        kept = d.gc_reuse[slot];
-        colour = false;
+      if (colour[u] && reuse && d.gc_island_chg[isl[u]] != itag) {
+        kept = d.gc_reuse[slot[u]];
+        colour[u] = false;
       }
-      if (colour || kept != BB_NONE) {
-        const uint32_t la = local_id(d, b.x), lb = local_id(d, b.y);
+      if (colour[u] || kept != BB_NONE) {
+        const uint32_t la = local_id(d, b[u].x), lb = local_id(d, b[u].y);
         uint32_t lo = min(la, lb), hi = max(la, lb);
-        const uint32_t pid = gc_hash(lo * 0x9e3779b9u + hi * 0x85ebca6bu + uint32_t(key) * 0xc2b2ae35u);
+        const uint32_t pid = gc_hash(lo * 0x9e3779b9u + hi * 0x85ebca6bu + uint32_t(kc[u].x) * 0xc2b2ae35u);
         d.gc_pid[m] = pid;
+        const bool da = fa[u] & BB_BODY_DYNAMIC, db = fb[u] & BB_BODY_DYNAMIC;
         // bit 2: neither body awake (both asleep or static); the sweeps have nothing to do there
-        const bool idle = !((fa & BB_BODY_DYNAMIC) && !(fa & BB_BODY_SLEEPING)) &&
-                          !((fb & BB_BODY_DYNAMIC) && !(fb & BB_BODY_SLEEPING));
-        d.gc_rec[m] = make_uint4(b.x, b.y, pid, (da ? 0u : 1u) | (db ? 0u : 2u) | (idle ? 4u : 0u));
+        const bool idle = !(da && !(fa[u] & BB_BODY_SLEEPING)) && !(db && !(fb[u] & BB_BODY_SLEEPING));
+        const uint32_t cls = BB_GC_CLASSES - min(max(uint32_t(kc[u].y), 1u), BB_GC_CLASSES);
+        d.gc_rec[m] = make_uint4(b[u].x, b[u].y, pid, (da ? 0u : 1u) | (db ? 0u : 2u) | (idle ? 4u : 0u) | cls << 3);
       }
-      d.gc_color[m] = kept != BB_NONE ? kept : colour ? BB_UNCOLORED : BB_RESTING;
+      if (slot[u] != BB_NONE) d.gc_color[m] = kept != BB_NONE ? kept : colour[u] ? BB_UNCOLORED : BB_RESTING;
       if (kept < BB_MAX_COLORS) used0 = max(used0, kept + 1u);
     }
-    const unsigned mask = __ballot_sync(0xFFFFFFFFu, colour);
-    if (mask) {
-      uint32_t off = 0;
-      if (lane == 0) off = atomicAdd(&c->gc_list_n[1], uint32_t(__popc(mask)));
-      off = __shfl_sync(0xFFFFFFFFu, off, 0);
-      if (colour) d.gc_list[1][off + __popc(mask & ((1u << lane) - 1u))] = m;
-    }
+    uint32_t mm[GC_UNROLL];
+#pragma unroll
+    for (int u = 0; u < GC_UNROLL; ++u) mm[u] = base + uint32_t(u) * stride + lane;
+    gc_append(&c->gc_list_n[1], d.gc_list[1], colour, mm);
   }
   used0 = __reduce_max_sync(0xFFFFFFFFu, used0);
   if (lane == 0 && used0) atomicMax(&c->gc_colors, used0);
@@ -436,10 +473,11 @@ __global__ void __launch_bounds__(BB_GC_THREADS, 1) k_edge_color(const DevState 
         ob[u] = live && !(rec[u].w & 2u) ? d.gc_owner[gc_owner_at(d, rec[u].y, col[u])] : 0ull;
       }
       uint32_t used = 0;  // colour + 1 of a committed manifold
+      bool keep[GC_UNROLL];
 #pragma unroll
       for (int u = 0; u < GC_UNROLL; ++u) {
-        bool keep = m[u] != BB_NONE;
-        if (keep && col[u] < BB_MAX_COLORS) {
+        keep[u] = m[u] != BB_NONE;
+        if (keep[u] && col[u] < BB_MAX_COLORS) {
           const bool sa = rec[u].w & 1u, sb = rec[u].w & 2u;
           const unsigned long long v = tag | gc_priority(rec[u].z, r);
           const bool wa = sa || oa[u] == v, wb = sb || ob[u] == v;
@@ -448,17 +486,11 @@ __global__ void __launch_bounds__(BB_GC_THREADS, 1) k_edge_color(const DevState 
             if (!sa) atomicOr(&d.gc_mask[rec[u].x], 1u << col[u]);
             if (!sb) atomicOr(&d.gc_mask[rec[u].y], 1u << col[u]);
             used = max(used, col[u] + 1u);
-            keep = false;
+            keep[u] = false;
           }
         }
-        const unsigned mask = __ballot_sync(0xFFFFFFFFu, keep);
-        if (mask) {
-          uint32_t off = 0;
-          if (lane == 0) off = atomicAdd(&c->gc_list_n[(r + 1) & 1], uint32_t(__popc(mask)));
-          off = __shfl_sync(0xFFFFFFFFu, off, 0);
-          if (keep) next[off + __popc(mask & ((1u << lane) - 1u))] = m[u];
-        }
       }
+      gc_append(&c->gc_list_n[(r + 1) & 1], next, keep, m);
       used = __reduce_max_sync(0xFFFFFFFFu, used);  // one colour-count update per warp
       if (lane == 0 && used) atomicMax(&c->gc_colors, used);
     }
@@ -474,17 +506,27 @@ __global__ void __launch_bounds__(BB_GC_THREADS, 1) k_edge_color(const DevState 
   // both asleep or static is also keyed 33: its sweep items would do nothing (both bodies are
   // frozen this substep).  Its colour (gc_color) is kept.
   uint32_t over = 0;
-  for (uint32_t m = tid; m < M; m += stride) {
-    uint32_t col = d.gc_color[m];
-    if (col == BB_UNCOLORED) ++over;
-    uint32_t key = col == BB_UNCOLORED ? BB_MAX_COLORS : col == BB_RESTING ? BB_MAX_COLORS + 1 : col;
-    if (key <= BB_MAX_COLORS && (reinterpret_cast<const uint32_t*>(d.gc_rec + m)[3] & 4u)) key = BB_MAX_COLORS + 1;
-    const uint32_t slot = d.man_slot[cur][m];
-    uint32_t cls = 0;
-    if (key < BB_MAX_COLORS) cls = BB_GC_CLASSES - min(max(uint32_t(d.m_keycc[cur][slot].y), 1u), BB_GC_CLASSES);
-    d.bucket_keys[0][m] = key * BB_GC_CLASSES + cls;
-    d.bucket_vals[0][m] = m;
-    d.gc_slot_color[cur][slot] = col;  // for the next substep's colour reuse
+  for (uint32_t m0 = tid; m0 < M; m0 += GC_UNROLL * stride) {
+    uint32_t col[GC_UNROLL], w[GC_UNROLL], slot[GC_UNROLL];
+#pragma unroll
+    for (int u = 0; u < GC_UNROLL; ++u) {
+      const uint32_t m = m0 + uint32_t(u) * stride;
+      if (m >= M) continue;
+      col[u] = d.gc_color[m];
+      w[u] = reinterpret_cast<const uint32_t*>(d.gc_rec + m)[3];  // not written for BB_RESTING, then not used
+      slot[u] = d.man_slot[cur][m];
+    }
+#pragma unroll
+    for (int u = 0; u < GC_UNROLL; ++u) {
+      const uint32_t m = m0 + uint32_t(u) * stride;
+      if (m >= M) continue;
+      if (col[u] == BB_UNCOLORED) ++over;
+      uint32_t key = col[u] == BB_UNCOLORED ? BB_MAX_COLORS : col[u] == BB_RESTING ? BB_MAX_COLORS + 1 : col[u];
+      if (key <= BB_MAX_COLORS && (w[u] & 4u)) key = BB_MAX_COLORS + 1;
+      d.bucket_keys[0][m] = key * BB_GC_CLASSES + (key < BB_MAX_COLORS ? w[u] >> 3 : 0u);
+      d.bucket_vals[0][m] = m;
+      d.gc_slot_color[cur][slot[u]] = col[u];  // for the next substep's colour reuse
+    }
   }
   if (over) atomicAdd(&c->gc_overflow, over);
   if (tid == 0) {
