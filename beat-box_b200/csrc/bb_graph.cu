@@ -56,8 +56,13 @@ __device__ __forceinline__ void st_relaxed_gpu(uint32_t* p, uint32_t v) {
 // the fixpoint every body points at the smallest id of its component -- the same roots as the
 // reference's link-to-lower union-find (islands.slang:153-213) -- after O(log diameter)
 // rounds, with no serial walk of a long chain by any one thread.
+// Bound by the latency of random loads (slot -> bodies -> parents): a thread keeps CC_UNROLL
+// chains in flight, and round 0 leaves the manifolds' bodies in compact order for the later rounds.
+// The stage on 1M boxes (3 M manifolds) fell 395 -> 294 us, on 1,024 worlds 167 -> 130 us; 2 and 8
+// entries gave 319 and 288 us, but 8 lost 1 to 7 % on worlds of up to 5,000 bodies.
 #define BB_CC_THREADS 512
 #define BB_CC_MAX_ROUNDS 96u
+#define CC_UNROLL 4  // entries a thread takes per trip
 __global__ void __launch_bounds__(BB_CC_THREADS, 1) k_components(const DevState d, int cur, uint32_t n) {
   DevCounters* c = d.ctr;
   const uint32_t tid = blockIdx.x * blockDim.x + threadIdx.x, stride = gridDim.x * blockDim.x;
@@ -66,6 +71,7 @@ __global__ void __launch_bounds__(BB_CC_THREADS, 1) k_components(const DevState 
   uint32_t* changed = c->round_flags;  // two alternating per-round flags (the AVBD colouring reuses them later)
   uint32_t ep = 0;
   uint32_t* parent = d.uf_parent;
+  uint2* pairs = reinterpret_cast<uint2*>(d.gc_rec);  // bodies of manifold m, from round 0 on (the colouring's scratch)
   // Start from the last substep's roots where that is exact.  A last-substep component whose
   // bodies are all dynamic and were not awake at either narrow phase (frozen bit 1) keeps every
   // one of its manifolds (two such bodies keep their poses, so their pairs and manifolds
@@ -95,22 +101,57 @@ __global__ void __launch_bounds__(BB_CC_THREADS, 1) k_components(const DevState 
   uint32_t r = 0;
   for (; r < BB_CC_MAX_ROUNDS; ++r) {
     uint32_t any = 0;
-    for (uint32_t m = tid; m < M; m += stride) {
-      const uint2 b = d.m_bodies[cur][d.man_slot[cur][m]];
-      const uint32_t pa = ld_relaxed_gpu(&parent[b.x]), pb = ld_relaxed_gpu(&parent[b.y]);
-      if (pa == BB_NONE || pb == BB_NONE || pa == pb) continue;
-      atomicMin(&parent[max(pa, pb)], min(pa, pb));
-      any = 1;
-    }
-    grid_sync(c, sync, ep);
-    for (uint32_t i = tid; i < n; i += stride) {
-      const uint32_t p = parent[i];
-      if (p == BB_NONE) continue;
-      const uint32_t pp = ld_relaxed_gpu(&parent[p]);
-      if (pp != p) {  // only this thread writes parent[i] in this pass
-        st_relaxed_gpu(&parent[i], pp);
+    for (uint32_t m0 = tid; m0 < M; m0 += CC_UNROLL * stride) {
+      uint2 b[CC_UNROLL];
+      uint32_t pa[CC_UNROLL], pb[CC_UNROLL];
+      if (r == 0u) {
+        uint32_t slot[CC_UNROLL];
+#pragma unroll
+        for (int u = 0; u < CC_UNROLL; ++u) {
+          const uint32_t m = m0 + uint32_t(u) * stride;
+          slot[u] = m < M ? d.man_slot[cur][m] : BB_NONE;
+        }
+#pragma unroll
+        for (int u = 0; u < CC_UNROLL; ++u)
+          b[u] = slot[u] != BB_NONE ? d.m_bodies[cur][slot[u]] : make_uint2(BB_NONE, BB_NONE);
+#pragma unroll
+        for (int u = 0; u < CC_UNROLL; ++u)
+          if (slot[u] != BB_NONE) pairs[m0 + uint32_t(u) * stride] = b[u];
+      } else {
+#pragma unroll
+        for (int u = 0; u < CC_UNROLL; ++u) {
+          const uint32_t m = m0 + uint32_t(u) * stride;
+          b[u] = m < M ? pairs[m] : make_uint2(BB_NONE, BB_NONE);
+        }
+      }
+#pragma unroll
+      for (int u = 0; u < CC_UNROLL; ++u) {
+        pa[u] = b[u].x != BB_NONE ? ld_relaxed_gpu(&parent[b[u].x]) : BB_NONE;
+        pb[u] = b[u].x != BB_NONE ? ld_relaxed_gpu(&parent[b[u].y]) : BB_NONE;
+      }
+#pragma unroll
+      for (int u = 0; u < CC_UNROLL; ++u) {
+        if (pa[u] == BB_NONE || pb[u] == BB_NONE || pa[u] == pb[u]) continue;
+        atomicMin(&parent[max(pa[u], pb[u])], min(pa[u], pb[u]));
         any = 1;
       }
+    }
+    grid_sync(c, sync, ep);
+    for (uint32_t i0 = tid; i0 < n; i0 += CC_UNROLL * stride) {
+      uint32_t p[CC_UNROLL], pp[CC_UNROLL];
+#pragma unroll
+      for (int u = 0; u < CC_UNROLL; ++u) {
+        const uint32_t i = i0 + uint32_t(u) * stride;
+        p[u] = i < n ? ld_relaxed_gpu(&parent[i]) : BB_NONE;
+      }
+#pragma unroll
+      for (int u = 0; u < CC_UNROLL; ++u) pp[u] = p[u] != BB_NONE ? ld_relaxed_gpu(&parent[p[u]]) : BB_NONE;
+#pragma unroll
+      for (int u = 0; u < CC_UNROLL; ++u)
+        if (pp[u] != p[u]) {  // only this thread writes parent[i] in this pass
+          st_relaxed_gpu(&parent[i0 + uint32_t(u) * stride], pp[u]);
+          any = 1;
+        }
     }
     if (any) atomicOr(&changed[r & 1], 1u);
     grid_sync(c, sync, ep);
@@ -256,10 +297,13 @@ __device__ __forceinline__ uint32_t gc_priority(uint32_t pid, uint32_t round) {
 //   commit: a manifold that won on both bodies takes the colour (:179-212).
 // Finally writes the (colour, manifold) keys of the bucket sort.
 // Persistent colouring kernel.  Each manifold's bodies, static bits and pair hash are packed
-// into one record up front (with the contact-count class for the keys), so a round touches rec -> body masks -> owner words only; the
-// grid barrier is the arrival-counter kind (counter 0 of the substep).
+// into one record up front (with the contact-count class for the keys), so a round touches rec ->
+// body masks -> owner words only; the grid barrier is the arrival-counter kind (counter 0 of the
+// substep).
 #define BB_GC_THREADS 1024
-#define GC_UNROLL 3  // entries a thread takes per trip (1M boxes: 1293 / 1138 / 1114 us at 2 / 3 / 4; 4 spills, small worlds lose 4 %)
+// Entries a thread takes per trip: colouring 1M boxes took 1293 / 1138 / 1114 us at 2 / 3 / 4; 4
+// spills, and small worlds lose 4 %.
+#define GC_UNROLL 3
 // Owner word of (body, colour), colour-major: a round's bids go mostly to the lowest free colours,
 // so the words in use (8 bytes per body for each colour bid) stay in L2, where a body-major
 // table (256 bytes per body) spread every round's random atomics over the whole table in DRAM.
