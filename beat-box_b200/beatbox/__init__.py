@@ -397,8 +397,8 @@ class World:
         _check(self.L.bb_step(self.h, ctypes.c_float(dt), substeps))
 
     def autotune(self, dt: float, substeps: int = 1, trial_steps: int = 2) -> dict:
-        """Time launch geometries / schedules on this world (each trial step advances it) and keep
-        the fastest; returns the chosen tunables."""
+        """Time launch geometries on this world (each trial step advances it) and keep the fastest;
+        returns the chosen tunables (schedule and pgs_stage_next come back as they were set)."""
         p = SolverParams()
         _check(self.L.bb_autotune(self.h, dt, substeps, trial_steps, ctypes.byref(p)))
         return dict(schedule=p.schedule, broad_threads=p.broad_threads, narrow_blocks_per_sm=p.narrow_blocks_per_sm,

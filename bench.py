@@ -65,7 +65,7 @@ def workload(args, n_bodies: int | None = None):
         name = (f"mixed_column_{nb // 1000}k: {nb} bodies (60% boxes / 40% spheres) in a "
                 f"60x60x200 m column, 5-wall container, dt=1/60, {SUBSTEPS} substeps, ")
     if args.solver == "pgs":
-        name += f"PGS_SOFT {pgs_iterations(args)} iterations ({args.schedule} schedule)"
+        name += f"PGS_SOFT {pgs_iterations(args)} iterations"
     else:
         name += "AVBD 4 iterations (beta=10)"
     return sc, name
@@ -733,7 +733,7 @@ def main():
                     help="pyramids: bodies/1000 box pyramids (default, 1M boxes); mixed_column: the 100k mixed "
                          "column; box_grid: the 1000-box grid; voxel_pile: concave voxel bodies")
     ap.add_argument("--schedule", default="barrier", choices=["dataflow", "barrier"],
-                    help="PGS schedule: per-body dataflow counters or a grid barrier per colour")
+                    help="accepted, no effect: the colour sweeps have one schedule (tagged velocities)")
     ap.add_argument("--mode", default="plain", choices=["plain", "batched", "served", "sort"],
                     help="plain: one world (default); batched: config-4 batch of independent worlds; "
                          "served: config-5 serving loop; sort: the a4 pair sort alone on --sort-keys keys")
