@@ -38,9 +38,6 @@ DT = 1.0 / 60.0
 SUBSTEPS = 4
 L2_BYTES = 126 * 1024 * 1024
 DEFAULT_BODIES = {"pyramids": 1_000_000, "mixed_column": 100_000, "box_grid": 1000, "voxel_pile": 20_000}
-# DRAM bytes (read + write) of one launch, from ncu captures of the same workloads; the capture
-# commands are in profiles/ (k_pgs_soft on the 100k mixed column at step ~298 of its run)
-SOLVER_TRAFFIC = {("mixed_column", 100_000): 114.5e6 + 24.1e6}
 
 
 def workload(args, n_bodies: int | None = None):
@@ -434,8 +431,7 @@ def run_ours(args, rank: int, world_size: int, local_rank: int):
     io_bytes = n * (12 + 16 + 12 + 12)
 
     # per-stage split and per-kernel rooflines on the timed steps
-    prof = profiled_window(bb, args, sc, local_rank, first, args.steps, peak_gbs,
-                           SOLVER_TRAFFIC.get((args.scene, args.bodies)) if args.solver == "pgs" else None)
+    prof = profiled_window(bb, args, sc, local_rank, first, args.steps, peak_gbs)
     stage = prof["stage_ms_per_substep"]
     dom = max(stage, key=stage.get) if stage else "solve"
     roof = dict(prof["rooflines"]["solve"])
@@ -458,8 +454,7 @@ def run_ours(args, rank: int, world_size: int, local_rank: int):
         wc.sync()
         ms2 = time_steps(torch, wc, args.steps, flush, dev)
         wc.close()
-        p2 = profiled_window(bb, a2, sc2, local_rank, f2, args.steps, peak_gbs,
-                             SOLVER_TRAFFIC.get((a2.scene, a2.bodies)))
+        p2 = profiled_window(bb, a2, sc2, local_rank, f2, args.steps, peak_gbs)
         extras["mixed_column_100k"] = {"workload": name2, "value": sc2["n"] * args.steps / (sum(ms2) / 1000.0),
                                        "unit": "body-steps/s", "ms_per_step": sum(ms2) / args.steps,
                                        "timed_steps": f"steps {f2}..{f2 + args.steps - 1} of the 600-step run",
