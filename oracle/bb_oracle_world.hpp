@@ -301,6 +301,12 @@ template <class R> class World {
         if (it != prev_pair_index.end()) {
           const Manifold<R>& old = prev_manifolds[it->second];
           update_from_old(m, old, old.a != m.a);
+          // The records hold the positions after matching, and a contact matched by distance the old
+          // one's features: matched by these here, it would move to the old position.
+          for (int c = 0; c < m.cc; ++c) {
+            const bb_contact_info& ci = inj_c[k * MAX_CONTACTS + c];
+            m.c[c].pos = Vec3<R>(R(ci.position[0]), R(ci.position[1]), R(ci.position[2]));
+          }
         }
       }
       manifolds.push_back(m);
