@@ -697,31 +697,74 @@ __device__ __forceinline__ void pgs_sweeps(const DevState& d, const Params& p, c
   }
 }
 
-// an item of the overflow bucket, run serially between grid barriers: tags stay as they are
-__device__ __forceinline__ void pgs_overflow_item(const DevState& d, const Params& p, uint32_t k, int mode,
-                                                  const PgsCoef& co) {
-  const uint4 rec = d.pgs_rec[k];
-  const uint32_t a = PGS_BODY(rec.x), b = PGS_BODY(rec.y), cc = rec.z & 15u;
-  PgsItem x = pgs_item_load(d, k);
-  pgs_item_coef(x, co);
-  const Sym3 IA = load_iw(d, a), IB = load_iw(d, b);
+// One sweep over the overflow bucket, items [o0, o1): serially in manifold order by one warp, between
+// grid barriers (plain loads and stores of the velocities; tags stay as they are).  Bound by the
+// chain of its items: 32 of them load at once, a lane each, then run one after the other, and an
+// item's velocities go to the later lanes with the same body by shuffles.  One thread that loaded
+// item after item and passed velocities through memory took 1.6 us per item of four contacts: 144
+// boxes on one dynamic plate (113 items, 84 sweeps per step) 19.7 -> 13.3 ms per step, a pile of 2,000
+// after one colouring round (3,443 items) 34.3 -> 17.5 ms.
+__device__ __forceinline__ void pgs_overflow(const DevState& d, const Params& p, uint32_t o0, uint32_t o1, int mode,
+                                             const PgsCoef& co) {
+  constexpr uint32_t ALL = 0xFFFFFFFFu;
+  const uint32_t lane = threadIdx.x & 31u;
   float4* vw = pgs_vw(d);
-  const float4 va4 = ld_tagged(vw + 2 * size_t(a)), wa4 = ld_tagged(vw + 2 * size_t(a) + 1);
-  const float4 vb4 = ld_tagged(vw + 2 * size_t(b)), wb4 = ld_tagged(vw + 2 * size_t(b) + 1);
-  float3 va = f3(va4), wa = f3(wa4), vb = f3(vb4), wb = f3(wb4);
-  for (uint32_t j = rec.w; j < rec.w + cc; ++j) {
-    float4 L = d.pgs_lam[j];
-    if (mode == 0) pgs_warm_contact<false>(x, d.c_r1[j], L, p.flags, IA, IB, va, wa, vb, wb);
-    else pgs_run_contact<false>(x, d.c_r1[j], pgs_tmass(d)[j], L, mode == 1, p.flags, IA, IB, va, wa, vb, wb);
-    d.pgs_lam[j] = L;
-  }
-  if (rec.x >> 31) {
-    st_tagged(vw + 2 * size_t(a), va, __float_as_uint(va4.w));
-    st_tagged(vw + 2 * size_t(a) + 1, wa, __float_as_uint(wa4.w));
-  }
-  if (rec.y >> 31) {
-    st_tagged(vw + 2 * size_t(b), vb, __float_as_uint(vb4.w));
-    st_tagged(vw + 2 * size_t(b) + 1, wb, __float_as_uint(wb4.w));
+  for (uint32_t k0 = o0; k0 < o1; k0 += 32u) {
+    const uint32_t count = min(32u, o1 - k0);
+    const uint4 rec = d.pgs_rec[k0 + min(lane, count - 1u)];
+    const uint32_t a = PGS_BODY(rec.x), b = PGS_BODY(rec.y), cc = lane < count ? rec.z & 15u : 0u;
+    PgsItem x = pgs_item_load(d, k0 + min(lane, count - 1u));
+    const Sym3 IA = load_iw(d, a), IB = load_iw(d, b);
+    float4 va4 = vw[2 * size_t(a)], wa4 = vw[2 * size_t(a) + 1], vb4 = vw[2 * size_t(b)], wb4 = vw[2 * size_t(b) + 1];
+    float4 A[BB_MAX_CONTACTS], L[BB_MAX_CONTACTS];
+    float2 B[BB_MAX_CONTACTS];
+#pragma unroll
+    for (int j = 0; j < BB_MAX_CONTACTS; ++j)
+      if (uint32_t(j) < cc) {
+        A[j] = d.c_r1[rec.w + j];
+        B[j] = pgs_tmass(d)[rec.w + j];
+        L[j] = d.pgs_lam[rec.w + j];
+      }
+    float3 va = f3(va4), wa = f3(wa4), vb = f3(vb4), wb = f3(wb4);
+    pgs_item_coef(x, co);
+    for (uint32_t l = 0; l < count; ++l) {
+      if (lane == l) {
+#pragma unroll 1
+        for (uint32_t j = 0; j < cc; ++j) {
+          if (mode == 0) {
+            pgs_warm_contact<false>(x, A[j], L[j], p.flags, IA, IB, va, wa, vb, wb);
+          } else {
+            float4 lam = L[j];
+            pgs_run_contact<false>(x, A[j], B[j], lam, mode == 1, p.flags, IA, IB, va, wa, vb, wb);
+            d.pgs_lam[rec.w + j] = lam;
+          }
+        }
+      }
+      __syncwarp();
+      auto from = [&](float3 v) {
+        return make_float3(__shfl_sync(ALL, v.x, int(l)), __shfl_sync(ALL, v.y, int(l)), __shfl_sync(ALL, v.z, int(l)));
+      };
+      const uint32_t la = __shfl_sync(ALL, rec.x, int(l)), lb = __shfl_sync(ALL, rec.y, int(l));
+      const float3 lva = from(va), lwa = from(wa), lvb = from(vb), lwb = from(wb);
+      if (la >> 31) {
+        if (rec.x == la) va = lva, wa = lwa;
+        if (rec.y == la) vb = lva, wb = lwa;
+      }
+      if (lb >> 31) {
+        if (rec.x == lb) va = lvb, wa = lwb;
+        if (rec.y == lb) vb = lvb, wb = lwb;
+      }
+    }
+    // (lanes that share a body hold the same velocities of it by now)
+    if (rec.x >> 31) {
+      vw[2 * size_t(a)] = f4(va, va4.w);
+      vw[2 * size_t(a) + 1] = f4(wa, wa4.w);
+    }
+    if (rec.y >> 31) {
+      vw[2 * size_t(b)] = f4(vb, vb4.w);
+      vw[2 * size_t(b) + 1] = f4(wb, wb4.w);
+    }
+    __syncwarp();
   }
 }
 
@@ -759,8 +802,7 @@ __global__ void __launch_bounds__(BB_PGS_THREADS, BB_PGS_PER_SM) k_pgs_soft(cons
     pgs_sweeps<PLAIN>(d, p, ft, co, s, e, warm, mid, dead);
     if (o0 != o1) {  // overflow bucket: serial, in manifold order
       grid_sync(d.ctr, sync, epoch);
-      if (tid == 0)
-        for (uint32_t k = o0; k < o1; ++k) pgs_overflow_item(d, p, k, s < warm ? 0 : s < mid ? 1 : 2, co);
+      if (tid < 32u) pgs_overflow(d, p, o0, o1, s < warm ? 0 : s < mid ? 1 : 2, co);
       grid_sync(d.ctr, sync, epoch);
     }
     s = e;
