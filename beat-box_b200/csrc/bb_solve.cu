@@ -317,6 +317,9 @@ __device__ __forceinline__ void pgs_integrate(const DevState& d, uint32_t i, flo
 #define BB_PGS_PER_SM 4
 #define BB_PGS_CLASSES BB_GC_CLASSES
 #define BB_PGS_PF 4  // contacts of an item loaded together
+// Sweeps between two grid barriers at most: a block that has no tiles, or is done with its own, waits
+// for the others at the next barrier, and this bounds that wait however many sweeps are asked for.
+#define BB_PGS_RUN 64u
 
 // body i's tagged velocities (linear, angular) next to each other, in row scratch this solver
 // does not use
@@ -798,11 +801,13 @@ __global__ void __launch_bounds__(BB_PGS_THREADS, BB_PGS_PER_SM) k_pgs_soft(cons
       integrated = true;
     }
     if (s >= last) break;
-    const uint32_t e = o0 != o1 ? s + 1u : s < mid ? mid : last;
+    const uint32_t e = o0 != o1 ? s + 1u : min(s < mid ? mid : last, s + BB_PGS_RUN);
     pgs_sweeps<PLAIN>(d, p, ft, co, s, e, warm, mid, dead);
     if (o0 != o1) {  // overflow bucket: serial, in manifold order
       grid_sync(d.ctr, sync, epoch);
       if (tid < 32u) pgs_overflow(d, p, o0, o1, s < warm ? 0 : s < mid ? 1 : 2, co);
+      grid_sync(d.ctr, sync, epoch);
+    } else if (e - s == BB_PGS_RUN) {
       grid_sync(d.ctr, sync, epoch);
     }
     s = e;

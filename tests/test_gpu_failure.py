@@ -59,6 +59,26 @@ def test_a_grid_barrier_wait_that_runs_out_is_reported_and_the_world_recovers():
         assert np.array_equal(a[k], b[k]), k
 
 
+def test_many_sweeps_do_not_run_into_the_wait_limit():
+    """8,000 sweeps of a few touching bodies in a world whose colour-sweep grid has many blocks without
+    work: a block that waits for the others waits for a bounded number of sweeps, so a wait limit far
+    below the whole phase's time (4096 polls) is not reached."""
+    sc = scenes.pile(40, seed=3)
+    w = bb.World(20_000)
+    w.add_scene(sc)
+    w.set_params(params(sc))
+    for _ in range(40):
+        w.step(DT, 4)
+    p = params(sc)
+    p.iterations = p.relax_iterations = 8000
+    w.set_params(p)
+    w.debug_wait_limit(4096)
+    w.step(DT / 4, 1)
+    w.sync()
+    st = w.stats()
+    assert st["error_flags"] == 0 and st["solved_manifolds"] > 20
+
+
 def test_capacity_overflow_regrows_and_equals_a_large_world():
     """A world created with one pair per body on overlapping boxes overflows its pair capacity;
     with auto-regrow bb_sync reallocates it with more pairs per body, restores the state from
