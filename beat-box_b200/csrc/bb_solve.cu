@@ -702,60 +702,62 @@ __device__ __forceinline__ void pgs_sweeps(const DevState& d, const Params& p, c
 
 // One sweep over the overflow bucket, items [o0, o1): serially in manifold order by one warp, between
 // grid barriers (plain loads and stores of the velocities; tags stay as they are).  Bound by the
-// chain of its items: 32 of them load at once, a lane each, then run one after the other, and an
-// item's velocities go to the later lanes with the same body by shuffles.  One thread that loaded
-// item after item and passed velocities through memory took 1.6 us per item of four contacts: 144
-// boxes on one dynamic plate (113 items, 84 sweeps per step) 19.7 -> 13.3 ms per step, a pile of 2,000
-// after one colouring round (3,443 items) 34.3 -> 17.5 ms.
+// chain of its items: BB_PGS_OVER of them load at once, a lane each, then run one after the other,
+// and an item's velocities go to the later lanes with the same body by shuffles.  One thread that
+// loaded item after item and passed velocities through memory took 1.6 us per item of four contacts:
+// 144 boxes on one dynamic plate (113 items, 84 sweeps per step) 19.8 -> 14.3 ms per step, a pile of
+// 2,000 after one colouring round (3,443 items) 34.3 -> 19.8 ms.  The contacts wait in shared memory:
+// in local arrays they cost the tiles' code 1.6 % (1,024 worlds), and 32 items' shared memory
+// takes L1 from the tiles' rows (0.4 %).
+#define BB_PGS_OVER 16u
 __device__ __forceinline__ void pgs_overflow(const DevState& d, const Params& p, uint32_t o0, uint32_t o1, int mode,
                                              const PgsCoef& co) {
+  __shared__ float4 A[BB_MAX_CONTACTS][BB_PGS_OVER], L[BB_MAX_CONTACTS][BB_PGS_OVER];
+  __shared__ float2 B[BB_MAX_CONTACTS][BB_PGS_OVER];
   constexpr uint32_t ALL = 0xFFFFFFFFu;
   const uint32_t lane = threadIdx.x & 31u;
   float4* vw = pgs_vw(d);
-  for (uint32_t k0 = o0; k0 < o1; k0 += 32u) {
-    const uint32_t count = min(32u, o1 - k0);
-    const uint4 rec = d.pgs_rec[k0 + min(lane, count - 1u)];
+  for (uint32_t k0 = o0; k0 < o1; k0 += BB_PGS_OVER) {
+    const uint32_t count = min(BB_PGS_OVER, o1 - k0), k = k0 + min(lane, count - 1u);
+    const uint4 rec = d.pgs_rec[k];
     const uint32_t a = PGS_BODY(rec.x), b = PGS_BODY(rec.y), cc = lane < count ? rec.z & 15u : 0u;
-    PgsItem x = pgs_item_load(d, k0 + min(lane, count - 1u));
+    PgsItem x = pgs_item_load(d, k);
     const Sym3 IA = load_iw(d, a), IB = load_iw(d, b);
-    float4 va4 = vw[2 * size_t(a)], wa4 = vw[2 * size_t(a) + 1], vb4 = vw[2 * size_t(b)], wb4 = vw[2 * size_t(b) + 1];
-    float4 A[BB_MAX_CONTACTS], L[BB_MAX_CONTACTS];
-    float2 B[BB_MAX_CONTACTS];
-#pragma unroll
-    for (int j = 0; j < BB_MAX_CONTACTS; ++j)
-      if (uint32_t(j) < cc) {
-        A[j] = d.c_r1[rec.w + j];
-        B[j] = pgs_tmass(d)[rec.w + j];
-        L[j] = d.pgs_lam[rec.w + j];
-      }
+    const float4 va4 = vw[2 * size_t(a)], wa4 = vw[2 * size_t(a) + 1], vb4 = vw[2 * size_t(b)], wb4 = vw[2 * size_t(b) + 1];
+#pragma unroll 1
+    for (uint32_t j = 0; j < cc; ++j) {
+      A[j][lane] = d.c_r1[rec.w + j];
+      B[j][lane] = pgs_tmass(d)[rec.w + j];
+      L[j][lane] = d.pgs_lam[rec.w + j];
+    }
     float3 va = f3(va4), wa = f3(wa4), vb = f3(vb4), wb = f3(wb4);
     pgs_item_coef(x, co);
     for (uint32_t l = 0; l < count; ++l) {
       if (lane == l) {
 #pragma unroll 1
         for (uint32_t j = 0; j < cc; ++j) {
+          float4 lam = L[j][lane];
           if (mode == 0) {
-            pgs_warm_contact<false>(x, A[j], L[j], p.flags, IA, IB, va, wa, vb, wb);
+            pgs_warm_contact<false>(x, A[j][lane], lam, p.flags, IA, IB, va, wa, vb, wb);
           } else {
-            float4 lam = L[j];
-            pgs_run_contact<false>(x, A[j], B[j], lam, mode == 1, p.flags, IA, IB, va, wa, vb, wb);
+            pgs_run_contact<false>(x, A[j][lane], B[j][lane], lam, mode == 1, p.flags, IA, IB, va, wa, vb, wb);
             d.pgs_lam[rec.w + j] = lam;
           }
         }
       }
       __syncwarp();
-      auto from = [&](float3 v) {
-        return make_float3(__shfl_sync(ALL, v.x, int(l)), __shfl_sync(ALL, v.y, int(l)), __shfl_sync(ALL, v.z, int(l)));
-      };
+      // (a dynamic body's bit 31 is set: only those are handed on)
       const uint32_t la = __shfl_sync(ALL, rec.x, int(l)), lb = __shfl_sync(ALL, rec.y, int(l));
-      const float3 lva = from(va), lwa = from(wa), lvb = from(vb), lwb = from(wb);
-      if (la >> 31) {
-        if (rec.x == la) va = lva, wa = lwa;
-        if (rec.y == la) vb = lva, wb = lwa;
+      float f[12] = {va.x, va.y, va.z, wa.x, wa.y, wa.z, vb.x, vb.y, vb.z, wb.x, wb.y, wb.z};
+#pragma unroll
+      for (int q = 0; q < 12; ++q) f[q] = __shfl_sync(ALL, f[q], int(l));
+      if (rec.x >> 31 && (rec.x == la || rec.x == lb)) {
+        va = rec.x == la ? make_float3(f[0], f[1], f[2]) : make_float3(f[6], f[7], f[8]);
+        wa = rec.x == la ? make_float3(f[3], f[4], f[5]) : make_float3(f[9], f[10], f[11]);
       }
-      if (lb >> 31) {
-        if (rec.x == lb) va = lvb, wa = lwb;
-        if (rec.y == lb) vb = lvb, wb = lwb;
+      if (rec.y >> 31 && (rec.y == la || rec.y == lb)) {
+        vb = rec.y == la ? make_float3(f[0], f[1], f[2]) : make_float3(f[6], f[7], f[8]);
+        wb = rec.y == la ? make_float3(f[3], f[4], f[5]) : make_float3(f[9], f[10], f[11]);
       }
     }
     // (lanes that share a body hold the same velocities of it by now)
