@@ -239,12 +239,13 @@ void orc_set_carry_frozen(void* hp, int on) {
 
 // The next substep's narrow phase uses these n manifolds (bb_manifold_info, pair order) and
 // their contacts (bb_contact_info, MAX_CONTACTS per manifold) as its geometry (no voxel keys).
-void orc_inject_manifolds(void* hp, const bb_manifold_info* m, const bb_contact_info* c, uint32_t n) {
+void orc_inject_manifolds(void* hp, const bb_manifold_info* m, const bb_contact_info* c, uint32_t n, int impulses) {
   Handle* h = static_cast<Handle*>(hp);
   auto set = [&](auto& w) {
     w.inj_m.assign(m, m + n);
     w.inj_c.assign(c, c + size_t(n) * MAX_CONTACTS);
     w.inj = true;
+    w.inj_impulses = impulses != 0;
   };
   if (h->dbl) set(*h->d);
   else set(*h->f);

@@ -32,7 +32,7 @@ template <class R> class World {
   // matching, anchors and tangent bases are still the oracle's own.
   std::vector<bb_manifold_info> inj_m;
   std::vector<bb_contact_info> inj_c;
-  bool inj = false;
+  bool inj = false, inj_impulses = false;  // injected contacts pending; with their impulses
 
   // products of the last substep (debug readback)
   std::vector<uint32_t> morton;       // code of body order[i]
@@ -268,7 +268,7 @@ template <class R> class World {
   // ------------------------------------------------------------------------------------
   // Narrow phase + warm start (collision_detection.slang:1514-1755).
   void narrow_from_injected() {
-    const bool warm = (p.flags & BB_SIM_WARM_STARTING) && !skip_warm_once;
+    const bool warm = (p.flags & BB_SIM_WARM_STARTING) && !skip_warm_once && !inj_impulses;
     manifolds.clear();
     for (size_t k = 0; k < inj_m.size(); ++k) {
       const bb_manifold_info& mi = inj_m[k];
@@ -289,6 +289,12 @@ template <class R> class World {
         ct.fp.out_ref = (ci.feature >> 8) & 0xFF;
         ct.fp.in_inc = (ci.feature >> 16) & 0xFF;
         ct.fp.out_inc = ci.feature >> 24;
+        if (inj_impulses) {
+          ct.ni = R(ci.normal_impulse);
+          ct.ti[0] = R(ci.tangent_impulse[0]);
+          ct.ti[1] = R(ci.tangent_impulse[1]);
+          ct.warm = ci.warm_start;
+        }
         m.c[c] = ct;
       }
       m.anchor_a = bodies[m.a].pos;
@@ -301,12 +307,6 @@ template <class R> class World {
         if (it != prev_pair_index.end()) {
           const Manifold<R>& old = prev_manifolds[it->second];
           update_from_old(m, old, old.a != m.a);
-          // The records hold the positions after matching, and a contact matched by distance the old
-          // one's features: matched by these here, it would move to the old position.
-          for (int c = 0; c < m.cc; ++c) {
-            const bb_contact_info& ci = inj_c[k * MAX_CONTACTS + c];
-            m.c[c].pos = Vec3<R>(R(ci.position[0]), R(ci.position[1]), R(ci.position[2]));
-          }
         }
       }
       manifolds.push_back(m);

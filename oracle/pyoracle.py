@@ -78,7 +78,7 @@ def lib():
         L.orc_step.argtypes = [P, ctypes.c_float, ctypes.c_uint32]
         L.orc_collide.argtypes = [P, ctypes.c_uint32]
         L.orc_skip_warm_starting_once.argtypes = [P]
-        L.orc_inject_manifolds.argtypes = [P, P, P, ctypes.c_uint32]
+        L.orc_inject_manifolds.argtypes = [P, P, P, ctypes.c_uint32, ctypes.c_int]
         L.orc_set_carry_frozen.argtypes = [P, ctypes.c_int]
         L.orc_read_state.argtypes = [P, P, P, P, P, P]
         L.orc_read_stats.argtypes = [P, ctypes.POINTER(StepStats)]
@@ -156,14 +156,18 @@ class Oracle:
     def skip_warm_starting_once(self):
         lib().orc_skip_warm_starting_once(self.h)
 
-    def inject_manifolds(self, manifolds: np.ndarray, contacts: np.ndarray):
+    def inject_manifolds(self, manifolds: np.ndarray, contacts: np.ndarray, impulses: bool = False):
         """The next substep's narrow phase takes this geometry (records in the library's
-        bb_manifold_info / bb_contact_info layouts, 8 contacts per manifold) instead of its own."""
+        bb_manifold_info / bb_contact_info layouts, 8 contacts per manifold) instead of its own.
+        impulses: the contacts' impulses are the ones the solve starts with (contacts read before it);
+        otherwise the oracle matches them with its own last contacts, as it does its own.  Records
+        of contacts that were matched already do not match the same way again (matching moves
+        positions and hands on features), so after a first substep give the impulses."""
         m = np.ascontiguousarray(manifolds)
         c = np.ascontiguousarray(contacts)
         assert c.size == 8 * m.size
         self._keep["inj"] = (m, c)
-        lib().orc_inject_manifolds(self.h, _ptr(m), _ptr(c), int(m.size))
+        lib().orc_inject_manifolds(self.h, _ptr(m), _ptr(c), int(m.size), 1 if impulses else 0)
 
     def state(self):
         pos = np.zeros((self.n, 3))

@@ -103,14 +103,23 @@ def tray(m):
 
 
 def follows_the_oracle(po, sc, p, substeps=2):
-    """Steps both through `substeps` (the second one starts with the first one's impulses)."""
+    """Steps both through `substeps`.  The second one starts with the first one's impulses, as the GPU
+    matched them: they are read from a narrow phase that runs ahead of the step and that the step
+    repeats."""
     w = bb.world_from_scene(sc, params=p)
     o = po.Oracle(sc, params=p, threads=os.cpu_count() or 1)
-    for _ in range(substeps):
+    for sub in range(substeps):
+        w.debug_collide(2)
+        before = w.debug_read("manifolds"), w.debug_read("contacts")
         w.step(DT / 4, 1)
         w.sync()
         man, con = w.debug_read("manifolds"), w.debug_read("contacts")
-        o.inject_manifolds(man, con)
+        for k in ("body_a", "body_b", "contact_count", "normal", "tangent"):
+            assert np.array_equal(before[0][k], man[k]), k
+        for k in ("position", "penetration", "feature", "warm_start"):
+            assert np.array_equal(before[1][k], con[k]), k
+        assert sub == 0 or before[1]["normal_impulse"].any()
+        o.inject_manifolds(man, before[1], impulses=True)
         o.step(DT / 4, 1)
         cnt, buf = o.debug_read(10)
         assert np.array_equal(man["color"], buf[:4 * cnt].view(np.uint32))
@@ -129,3 +138,77 @@ def test_a_body_with_more_manifolds_than_colours(oracle_lib, m):
     sc = tray(m)
     st, _ = follows_the_oracle(oracle_lib, sc, params(oracle_lib, sc))
     assert st["graph_color_overflow"] == m * m + 1 - 32
+
+
+def settled_on_the_gpu(sc, p, steps):
+    """The scene in the state it has after `steps` steps, every body awake."""
+    w = bb.world_from_scene(sc, params=p)
+    for _ in range(steps):
+        w.step(DT, 4)
+    st = w.read_state()
+    w.close()
+    return dict(sc, **{k: np.ascontiguousarray(v, np.float32) for k, v in st.items()})
+
+
+def touching_pyramids(n_pyramids, boxes_per):
+    sc = scenes.pyramids(n_pyramids=n_pyramids, boxes_per=boxes_per, seed=0)
+    y = sc["pos"][1:, 1]
+    y[...] = 0.4995 + 0.9995 * np.round((y - 0.5) / 1.001)
+    return jolted(sc)
+
+
+@pytest.mark.parametrize("name", ["pile_20000", "pyramids_20x1000", "pile_600_two_rounds"])
+def test_sweeps_follow_the_oracle(oracle_lib, name):
+    """Piles with contacts of one to eight points, and pyramids, on a grid of 320 warps: a warp of the
+    larger ones takes several tiles of 32 manifolds per sweep.  Two colouring rounds leave
+    hundreds of manifolds to the overflow bucket, in more than one of its chunks."""
+    if name.startswith("pile"):
+        n = int(name.split("_")[1])
+        sc = scenes.pile(n, seed=4, sphere_fraction=0.3)
+        p = params(oracle_lib, sc, **(dict(gc_rounds=2) if n == 600 else {}))
+        sc = jolted(settled_on_the_gpu(sc, params(oracle_lib, sc), 40))
+    else:
+        sc = touching_pyramids(20, 1000)
+        p = params(oracle_lib, sc)
+    st, man = follows_the_oracle(oracle_lib, sc, p)
+    if name == "pile_600_two_rounds":
+        assert st["graph_color_overflow"] > 300
+    else:
+        assert st["solved_manifolds"] > 2 * 320 * 32 and st["graph_color_overflow"] == 0
+    if name.startswith("pile"):
+        assert man["contact_count"].min() == 1 and man["contact_count"].max() > 6
+
+
+@pytest.mark.parametrize("name", ["mixed_3000", "pyramids_20x1000"])
+def test_the_grid_does_not_change_the_bits(oracle_lib, name):
+    """A world's capacity sets the grid: with room for 80,000 bodies the sweeps run on every SM, sized
+    to the scene on a few, and each warp takes other tiles.  The bits are the same."""
+    sc = touching_pyramids(20, 1000) if name != "mixed_3000" else scenes.mixed_column(n_bodies=3000, seed=2)
+    steps = 5 if name != "mixed_3000" else 300  # (the column is in the air for the first 200)
+    outs = []
+    for capacity in (int(sc["n"]), 80_000):
+        w = bb.World(capacity, pairs_per_body=16)
+        w.add_scene(sc)
+        w.set_params(params(oracle_lib, sc))
+        for _ in range(steps):
+            w.step(DT, 4)
+        assert w.stats()["error_flags"] == 0 and w.stats()["solved_manifolds"] > 500
+        outs.append(w.read_state())
+        w.close()
+    for k in outs[0]:
+        assert np.array_equal(outs[0][k], outs[1][k]), k
+
+
+def test_two_runs_on_the_whole_gpu_give_the_same_bits(oracle_lib):
+    """200,000 boxes, over 400,000 manifolds: some 15 tiles per warp and sweep on every SM."""
+    sc = touching_pyramids(200, 1000)
+    outs = []
+    for _ in range(2):
+        w = bb.world_from_scene(sc, params=params(oracle_lib, sc))
+        for _ in range(4):
+            w.step(DT, 4)
+        outs.append(w.read_state())
+        assert w.stats()["error_flags"] == 0 and w.stats()["manifold_count"] > 400_000
+        w.close()
+    for k in outs[0]:
+        assert np.array_equal(outs[0][k], outs[1][k]), k
