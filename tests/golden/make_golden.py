@@ -4,6 +4,9 @@ The reference repository ships no golden vectors, so these fixtures are produced
 (the CPU restatement of the reference step) and pin it against unintended changes; the CUDA
 library is compared with the same oracle in the GPU tests.  Re-run after a deliberate change to
 the restated algorithm:  python tests/golden/make_golden.py
+
+colour_sweeps.npz holds the library's own bits and is written only when it is named, on a machine
+with a GPU:  python tests/golden/make_golden.py colour_sweeps
 """
 import os
 import sys
@@ -60,7 +63,25 @@ def generate(name):
     return out
 
 
+def colour_sweeps():
+    """Settled piles and the states one substep of the library makes of them."""
+    sys.path.insert(0, os.path.dirname(HERE))
+    import test_gpu_colour_sweeps as t
+
+    piles = {n: t.settled_pile(pyoracle, n) for n in sorted({n for n, _ in t.CASES})}
+    out = {f"settled_{k}_{n}": v for n, st in piles.items() for k, v in st.items()}
+    for i, (n, kw) in enumerate(t.CASES):
+        got, st = t.run_case(pyoracle, n, kw, piles[n])
+        assert st["error_flags"] == 0
+        out.update({f"{k}_{i}": v for k, v in got.items()})
+    return out
+
+
 def main():
+    if "colour_sweeps" in sys.argv[1:]:
+        np.savez_compressed(os.path.join(HERE, "colour_sweeps.npz"), **colour_sweeps())
+        print("wrote colour_sweeps")
+        return
     for name in CASES:
         np.savez_compressed(os.path.join(HERE, f"{name}.npz"), **generate(name))
         print("wrote", name)
