@@ -2,9 +2,10 @@
 runs out is reported by bb_sync as BB_E_DEVICE_LIMIT, and the world steps normally afterwards.
 
 The wait is made to run out by a block that never arrives: bb_debug_wait_limit's abandon switch
-makes the last block of the colour-sweep kernel leave before its first grid barrier, and a short
-wait limit (4096 polls, a few milliseconds) bounds every other block's wait for it.  Nothing
-spins without a bound and no kernel traps.  Reference counterpart: the bounded walks of
+makes the last block of the colour-sweep kernel leave at once, and a short wait limit (4096 polls, a
+few milliseconds) bounds every other block's wait for it: for a body that the block should have
+updated, or at a grid barrier where the block had no work.  Nothing spins without a bound and no
+kernel traps.  Reference counterpart: the bounded walks of
 avbd.slang:559, collision_detection.slang:921 and LBVH.slang:226,278, which stop without
 reporting."""
 import numpy as np
@@ -26,19 +27,30 @@ def params(sc):
     return p
 
 
-def test_a_grid_barrier_wait_that_runs_out_is_reported_and_the_world_recovers():
-    sc = scenes.pile(20_000, seed=3)  # 10k items per colour at most: a colour-sweep grid of many blocks
-    w = bb.world_from_scene(sc, params=params(sc))
-    for _ in range(3):
+SITE_BODY, SITE_SWEEP_BARRIER = 2, 16 + 1  # bb_step_stats.error_site
+
+
+@pytest.mark.parametrize("site", [SITE_BODY, SITE_SWEEP_BARRIER])
+def test_a_wait_that_runs_out_is_reported_and_the_world_recovers(site):
+    """SITE_BODY: a pile with more tiles than the grid has warps, so the block that leaves owns some, and
+    blocks with later ones wait for its bodies.  SITE_SWEEP_BARRIER: a few touching bodies, one tile
+    per colour, none of them the last block's; the others wait for it at the barrier."""
+    sc = scenes.pile(20_000 if site == SITE_BODY else 40, seed=3)
+    w = bb.World(20_001)
+    w.add_scene(sc)
+    w.set_params(params(sc))
+    for _ in range(40):
         w.step(DT, 4)
     w.sync()
-    assert w.stats()["manifold_count"] > 1000
+    manifolds = w.stats()["solved_manifolds"]  # the grid has 160 blocks of 2 warps
+    assert manifolds > 32 * 320 if site == SITE_BODY else 0 < manifolds < 159
     w.debug_wait_limit(4096, abandon_block=True)
     w.step(DT, 1)
     with pytest.raises(bb.BeatboxError) as e:
         w.sync()
     assert e.value.code == bb.E_DEVICE_LIMIT
     assert w.stats()["error_flags"] & ERRF_SPIN_LIMIT
+    assert w.stats()["error_site"] == site
     # the error is sticky until the world is cleared
     w.debug_wait_limit(0, abandon_block=False)
     with pytest.raises(bb.BeatboxError):
