@@ -53,8 +53,7 @@ struct DevCounters {
   uint32_t stick;
   uint32_t error_flags;    // sticky until read
   uint32_t gc_epoch;       // colouring round epoch (never reset)
-  uint32_t barrier_count;  // grid barrier
-  uint32_t barrier_gen;
+  uint32_t unused[2];  // (kept: the counters are part of saved states)
   uint32_t bounds_min[3];  // BB_BOUNDS_AUTO: ordered-float min/max of positions
   uint32_t bounds_max[3];
   uint32_t avbd_body_count;
@@ -164,7 +163,7 @@ struct DevState {
   uint32_t* island_start;  // per-island path: first sorted manifold of each island
   // colouring
   uint32_t* gc_color;    // per compact manifold
-  uint32_t* gc_pid;      // pair-identity hash
+  uint32_t* gc_pid;      // not used (kept: the arrays are the layout of saved states)
   uint32_t* gc_choice;
   uint4* gc_rec;         // per compact manifold: body a, body b, pair hash, bits 0..2 static / idle, class << 3
   uint32_t* gc_list[2];  // manifolds still uncoloured after a round (alternating)
@@ -173,7 +172,7 @@ struct DevState {
   unsigned long long* gc_owner; // 32 colours x (body capacity + 1) bodies: (epoch << 32) | priority
   uint32_t *bucket_keys[2], *bucket_vals[2]; // colour sort of manifolds / bodies
   uint32_t* bucket_start; // 34 + 32*L entries
-  uint32_t* colour_awake; // not used (kept: the arrays are the layout of saved states)
+  uint32_t* colour_awake; // not used (kept as gc_pid)
   // colour reuse: an island whose manifolds (bodies and key) are exactly last substep's keeps
   // last substep's colours (the colouring of an island depends on that set alone)
   uint32_t* gc_slot_color[2]; // per manifold slot of each buffer: the colour the colouring gave it
@@ -345,11 +344,10 @@ __device__ __forceinline__ Sym3 body_world_inv_inertia(const float4* iinv, const
 
 // Sites of bounded waits, recorded in DevCounters::error_site by the first one that gives up
 // (bb_step_stats.error_site): the sort's and the scan's look-backs, the PGS_SOFT sweeps' wait for a body,
-// the generation barrier, and BB_SITE_GRID + k for the grid barrier on sync_count[k] (0 edge colouring, 1
-// PGS_SOFT, 2 AVBD colouring, 3..5 AVBD solve phases, 7 connected components).
+// and BB_SITE_GRID + k for the grid barrier on sync_count[k] (0 edge colouring, 1 PGS_SOFT, 2 AVBD
+// colouring, 3..5 AVBD solve phases, 7 connected components).  3 named a barrier that is gone.
 #define BB_SITE_SORT 1u
 #define BB_SITE_FLOW 2u
-#define BB_SITE_GEN_BARRIER 3u
 #define BB_SITE_SCAN 4u
 #define BB_SITE_GRID 16u
 __device__ __forceinline__ void raise_error(DevCounters* c, uint32_t bit) { atomicOr(&c->error_flags, bit); }
@@ -377,9 +375,6 @@ __device__ __forceinline__ float ord2f(uint32_t v) {
 }
 
 // ---- grid barrier for persistent cooperative kernels ------------------------------------
-// Sense by generation counter; the spin is bounded: on timeout the block raises
-// BB_ERRF_SPIN_LIMIT and every later barrier returns at once (results are then invalid and
-// the host reports BB_E_DEVICE_LIMIT).
 __device__ __forceinline__ uint32_t ld_acquire_gpu(const uint32_t* p) {
   uint32_t v;
   asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
@@ -401,30 +396,12 @@ __device__ __forceinline__ bool spin_gave_up(DevCounters* c, uint32_t spins, uin
   return (ld_acquire_gpu(&c->error_flags) & BB_ERRF_SPIN_LIMIT) != 0;
 }
 
-__device__ __forceinline__ void grid_barrier(DevCounters* c) {
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    uint32_t g = ld_acquire_gpu(&c->barrier_gen);
-    fence_acq_rel_gpu();  // publish this block's writes (cumulative over the CTA barrier)
-    uint32_t arrived = atomicAdd(&c->barrier_count, 1u);
-    if (arrived == gridDim.x - 1) {
-      c->barrier_count = 0;
-      fence_acq_rel_gpu();
-      atomicAdd(&c->barrier_gen, 1u);
-    } else {
-      uint32_t spins = 0;
-      while (ld_acquire_gpu(&c->barrier_gen) == g)
-        if (spin_gave_up(c, ++spins, BB_SITE_GEN_BARRIER)) break;
-    }
-    fence_acq_rel_gpu();
-  }
-  __syncthreads();
-}
-
-// Grid barrier on a monotonic arrival counter that is zero when the kernel starts (one counter
-// per persistent launch of a substep): block thread 0 publishes the block's writes and adds one
-// without waiting for a reply, then polls until all blocks of this epoch arrived.  Two round
-// trips fewer than the generation barrier above (no generation read, no atomic reply).
+// Monotonic arrival counter that is zero when the kernel starts (one counter per persistent launch
+// of a substep): block thread 0 publishes the block's writes and adds one without waiting for a
+// reply, then polls until all blocks of this epoch arrived.  Two round trips fewer than a
+// generation barrier (no generation read, no atomic reply).  The spin is bounded: on timeout the
+// block raises BB_ERRF_SPIN_LIMIT and every later barrier returns at once (results are then
+// invalid and the host reports BB_E_DEVICE_LIMIT).
 __device__ __forceinline__ void red_relaxed_add(uint32_t* p, uint32_t v) {
   asm volatile("red.relaxed.gpu.global.add.u32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
 }
@@ -435,27 +412,6 @@ __device__ __forceinline__ void grid_sync(DevCounters* c, uint32_t* count, uint3
   if (threadIdx.x == 0) {
     fence_acq_rel_gpu();  // release this block's writes (cumulative over the CTA barrier)
     red_relaxed_add(count, 1u);
-    const uint32_t target = epoch * gridDim.x;
-    uint32_t spins = 0;
-    while (ld_acquire_gpu(count) < target)
-      if (spin_gave_up(c, ++spins, BB_SITE_GRID + uint32_t(count - c->sync_count))) break;
-  }
-  __syncthreads();
-}
-
-// grid_sync split in two: arrive publishes this block's writes and counts it in; wait returns
-// once every block of the epoch has arrived.  Work placed between them must neither read what
-// other blocks write in this epoch nor write what they read.
-__device__ __forceinline__ void grid_arrive(uint32_t* count, uint32_t& epoch) {
-  __syncthreads();
-  ++epoch;
-  if (threadIdx.x == 0 && gridDim.x > 1) {
-    fence_acq_rel_gpu();
-    red_relaxed_add(count, 1u);
-  }
-}
-__device__ __forceinline__ void grid_wait(DevCounters* c, const uint32_t* count, uint32_t epoch) {
-  if (threadIdx.x == 0 && gridDim.x > 1) {
     const uint32_t target = epoch * gridDim.x;
     uint32_t spins = 0;
     while (ld_acquire_gpu(count) < target)

@@ -420,7 +420,6 @@ __global__ void __launch_bounds__(BB_GC_THREADS, 1) k_edge_color(const DevState 
         const uint32_t la = local_id(d, b[u].x), lb = local_id(d, b[u].y);
         uint32_t lo = min(la, lb), hi = max(la, lb);
         const uint32_t pid = gc_hash(lo * 0x9e3779b9u + hi * 0x85ebca6bu + uint32_t(kc[u].x) * 0xc2b2ae35u);
-        d.gc_pid[m] = pid;
         const bool da = fa[u] & BB_BODY_DYNAMIC, db = fb[u] & BB_BODY_DYNAMIC;
         // bit 2: neither body awake (both asleep or static); the sweeps have nothing to do there
         const bool idle = !(da && !(fa[u] & BB_BODY_SLEEPING)) && !(db && !(fb[u] & BB_BODY_SLEEPING));

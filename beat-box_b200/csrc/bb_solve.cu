@@ -20,17 +20,9 @@
 
 // ---------------------------------------------------------------------------------------
 // PGS_SOFT
-struct BodyVel {
-  float3 v, w;
-};
-
 __device__ __forceinline__ Sym3 load_iw(const DevState& d, uint32_t i) {
   float4 a = d.iw[2 * i], b = d.iw[2 * i + 1];
   return Sym3{a.x, a.y, a.z, a.w, b.x, b.y};
-}
-__device__ __forceinline__ void store_iw(const DevState& d, uint32_t i, const Sym3& s) {
-  d.iw[2 * i] = make_float4(s.xx, s.xy, s.xz, s.yy);
-  d.iw[2 * i + 1] = make_float4(s.yz, s.zz, 0.f, 0.f);
 }
 __device__ __forceinline__ bool awake(uint32_t f) { return (f & BB_BODY_DYNAMIC) && !(f & BB_BODY_SLEEPING); }
 
@@ -315,7 +307,6 @@ __device__ __forceinline__ void pgs_integrate(const DevState& d, uint32_t i, flo
 // the contact's position minus the two anchors, as the pre-step forms them.
 #define BB_PGS_THREADS 64
 #define BB_PGS_PER_SM 4
-#define BB_PGS_CLASSES BB_GC_CLASSES
 #define BB_PGS_PF 4  // contacts of an item loaded together
 // Sweeps between two grid barriers at most: a block that has no tiles, or is done with its own, waits
 // for the others at the next barrier, and this bounds that wait however many sweeps are asked for.
@@ -385,12 +376,14 @@ __device__ __forceinline__ uint32_t pgs_tile_item(const PgsTiles& ft, uint32_t t
 // of the item)
 #define PGS_BODY(x) ((x) & 0x7FFFFFFFu)
 
-// before the sweeps, per body: world inverse inertia, tagged velocities, no colours yet
-__global__ void k_pgs_bodies(const DevState d, uint32_t n, Params p) {
+// before a solve, per body: world inverse inertia and, for the colour sweeps, tagged velocities and no
+// colours yet
+__global__ void k_pgs_bodies(const DevState d, uint32_t n, Params p, bool sweeps) {
   const bool tq = p.quirks & BB_QUIRK_INERTIA_TRANSPOSE;
   float4* vw = pgs_vw(d);
   for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
     pgs_world_inertia(d, i, tq);
+    if (!sweeps) continue;
     d.flow_counter[i] = 0u;
     vw[2 * size_t(i)] = f4(f3(d.vel[i]), 0.f);
     vw[2 * size_t(i) + 1] = f4(f3(d.omega[i]), 0.f);
@@ -882,7 +875,7 @@ void bb_solve_pgs_soft(cudaStream_t s, const DevState& d, const Params& p, uint3
   if (n == 0) return;
   const int T = BB_THREADS;
   const uint32_t blocks = (n + T - 1) / T;
-  k_pgs_bodies<<<blocks, T, 0, s>>>(d, n, p);
+  k_pgs_bodies<<<blocks, T, 0, s>>>(d, n, p, true);
   k_pgs_count<<<sms * 8, T, 0, s>>>(d, cur);
   bb_launch_scan(s, d.pgs_cnt, d.pgs_coff, &d.bucket_start[BB_MAX_COLORS + 1], d.pair_capacity, &d.ctr->pgs_contacts,
                  sc.scan_status + 4 * size_t(sc.scan_tiles), sc.scan_tile_ctr + 4, d.ctr);
@@ -1064,7 +1057,7 @@ void bb_solve_islands(cudaStream_t s, const DevState& d, const Params& p, uint32
   if (n == 0) return;
   const int T = BB_THREADS;
   const uint32_t blocks = (n + T - 1) / T;
-  k_pgs_bodies<<<blocks, T, 0, s>>>(d, n, p);  // world inverse inertia of every body
+  k_pgs_bodies<<<blocks, T, 0, s>>>(d, n, p, false);
   k_island_keys<<<sms * 8, T, 0, s>>>(d, cur);
   uint32_t* keys[2] = {d.bucket_keys[0], d.bucket_keys[1]};
   uint32_t* vals[2] = {d.bucket_vals[0], d.bucket_vals[1]};

@@ -309,7 +309,6 @@ __global__ void k_begin_substep(DevCounters* c) {
   c->avbd_colors = 0;
   c->avbd_violations = 0;
   c->stick = 0;
-  c->barrier_count = 0;
   c->round_flags[0] = 0;
   c->round_flags[1] = 0;
   c->heavy_n = 0;
