@@ -462,8 +462,8 @@ class World:
         _check(self.L.bb_debug_collide(self.h, stage))
 
     def debug_wait_limit(self, polls: int, abandon_block: bool = False):
-        """Bound of the persistent kernels' grid-barrier waits (0 = default); abandon_block makes
-        the colour-sweep kernel's last block leave so the other blocks' waits run out."""
+        """Bound of the persistent kernels' waits, in polls (0 = default); abandon_block makes the
+        colour-sweep kernel's last block leave so the other blocks' waits run out."""
         _check(self.L.bb_debug_wait_limit(self.h, polls, 1 if abandon_block else 0))
 
     def set_auto_regrow(self, max_pairs_per_body: int):

@@ -892,7 +892,10 @@ __device__ __forceinline__ void np_store(const DevState& d, const Params& p, int
 // -> 2.29 ms, 1,024 batched worlds 1.35 -> 1.07 ms, 20k mixed pile 188 -> 146 us, 1,000 boxes 114 ->
 // 94 us.  Tried and slower: pairs sorted by separating axis before the clip (2.98 ms).
 #define BB_NARROW_THREADS 128
-#define BB_NARROW_PER_SM 6  // 80 registers (some spilled): the second half waits on memory
+// 80 registers (some spilled): the second half waits on memory.  The compiler contracts box_box's plain
+// expressions as it sees fit: at 114 registers the last bits of some contacts differed, so stored
+// bits (tests/golden/colour_sweeps.npz) hang on this bound and on the compiler.
+#define BB_NARROW_PER_SM 6
 #define NP_GROUP 8
 static_assert(NP_GROUP == BB_MAX_CONTACTS, "a lane per contact");
 // a touching pair between the halves: normal and contact count | key << 8; position of a and slot;

@@ -271,6 +271,9 @@ __global__ void __launch_bounds__(kSortThreads, 2) k_onesweep(const uint32_t* __
   // digit, and the lowest of them advances the warp's count of the digit and hands the old count to
   // the others by a shuffle.  kSortMasks keys of a thread are in flight, each with mask words of its own
   // (they lie where the reordered keys and values go later).  rank keeps the digit in its top 8 bits.
+  // The multisplit is Ashkiani et al.'s (GPU Multisplit, 2016) and the one-sweep structure Adinets and
+  // Merrill's (Onesweep, 2022); or-ing lane bits where ballots would find a digit's lanes is a known
+  // variant of the former.
   uint32_t* masks = s_keys + warp * (kSortMasks * 256);
 #pragma unroll
   for (int i = 0; i < kSortMasks * 256 / 32; ++i) masks[i * 32 + lane] = 0u;

@@ -757,9 +757,11 @@ bb_status bb_world_create(const bb_world_desc* desc, void** out_world) {
     return st;
   }
   // Persistent grids sized to the world's capacity: about one thread per item of the largest
-  // colour (~half the bodies) for the sweeps, about one per body for colouring and components.
-  // A small world then runs on a block or two (its barriers become CTA barriers) and leaves
-  // the rest of the GPU to other worlds' streams.  Results do not depend on the grid.
+  // colour (~half the bodies) for the PGS_SOFT sweeps (four blocks of 64 at least) and the AVBD
+  // colouring, about one per body for the AVBD sweeps, edge colouring and components.  A small
+  // world then runs on a few blocks (colouring and components on one, whose barriers are CTA
+  // barriers) and leaves the rest of the GPU to other worlds' streams.  Results do not depend on
+  // the grid.
   auto fit = [](int max_blocks, uint64_t items, int threads) {
     return int(std::max<uint64_t>(1, std::min<uint64_t>(uint64_t(max_blocks), (items + threads - 1) / threads)));
   };
@@ -1859,8 +1861,7 @@ const uint32_t* bb_world_error_site_word(void* world) { return world ? &W(world)
 
 
 // ---- autotuner ------------------------------------------------------------------------------
-// Coordinate descent over the launch-geometry fields and the colour-sweep schedule of
-// bb_solver_params.  Every candidate computes bit-identical results, so the trial steps are
+// Coordinate descent over the launch-geometry fields of bb_solver_params.  Every candidate computes bit-identical results, so the trial steps are
 // ordinary steps of the world (they advance it; call this in place of warm-up steps).  Each
 // candidate gets one untimed step (graph capture) and `trial_steps` steps timed with CUDA
 // events on the world's stream.

@@ -133,7 +133,7 @@ typedef struct bb_solver_params {
   uint32_t avbd_color_rounds;  /* 16 */
   uint32_t avbd_shock_layers;  /* 12 */
   uint32_t avbd_post_stab_sweeps; /* 4 */
-  /* execution schedule of the colour sweeps (results are identical either way) */
+  /* no effect (kept for callers that set it; see the colour-sweep schedules above) */
   uint32_t schedule;           /* BB_SCHEDULE_* (default BB_SCHEDULE_COLOUR_BARRIER) */
   /* launch geometry (results are identical for every value; 0 = default; bb_autotune picks) */
   uint32_t broad_threads;        /* broad-phase block size: 32, 64 or 128 (default 128) */
@@ -375,12 +375,12 @@ bb_status bb_debug_collide(void* world, uint32_t stage);
  * receives the element count; at most max_bytes are written. */
 bb_status bb_debug_read(void* world, uint32_t which, void* dst, uint64_t max_bytes, uint64_t* count);
 
-/* Bounded device waits, for tests of the failure path.  polls: how many polls a grid-barrier
- * wait of this world's persistent kernels makes before it gives up (0 = the default, 2^22),
- * raising BB_ERRF_SPIN_LIMIT so that bb_sync returns BB_E_DEVICE_LIMIT.  abandon_block = 1
- * makes the last block of the PGS_SOFT colour-sweep kernel leave before its first grid barrier
- * (when the kernel runs on more than one block), so the other blocks wait for a block that
- * never arrives until their bounded waits give up; the step's results are then undefined, and
+/* Bounded device waits, for tests of the failure path.  polls: how many polls a wait of this
+ * world's persistent kernels (at a grid barrier, or of the colour sweeps for a body) makes before
+ * it gives up (0 = the default, 2^22), raising BB_ERRF_SPIN_LIMIT so that bb_sync returns
+ * BB_E_DEVICE_LIMIT.  abandon_block = 1 makes the last block of the PGS_SOFT colour-sweep kernel
+ * leave at once (when the kernel runs on more than one block), so the other blocks wait for it,
+ * or for bodies that it should have updated, until their bounded waits give up; the step's results are then undefined, and
  * bb_world_clear (which also clears the error bits) makes the world usable again.  No
  * counterpart in the reference: its bounded loops (avbd.slang:559, collision_detection.slang:921,
  * LBVH.slang:226,278) stop without reporting. */
@@ -461,12 +461,10 @@ bb_status bb_radix_sort_pairs_static(const uint32_t* keys_in, const uint32_t* va
  * sort passes clamp silently, LBVH.slang:34-152). */
 bb_status bb_radix_sort_error_flags(uint32_t static_scratch, void* stream, uint32_t* error_flags);
 
-/* Pick the launch geometry of this world by timing candidates
- * (coordinate descent over bb_solver_params.broad_threads, narrow_blocks_per_sm;
- * pgs_stage_next; each candidate timed between two runs of the incumbent).  All candidates
- * give bit-identical results, so the trial steps are ordinary steps (about 21 x
- * (trial_steps + 1) of them): use it in place of warm-up.  The
- * winner is set on the world and copied to *chosen (may be NULL).  The reference has no
+/* Pick the launch geometry of this world by timing candidates (coordinate descent over
+ * bb_solver_params.broad_threads and narrow_blocks_per_sm; each candidate timed between two
+ * runs of the incumbent).  All candidates give bit-identical results, so the trial steps are
+ * ordinary steps (15 to 21 x (trial_steps + 1) of them): use it in place of warm-up.  The winner is set on the world and copied to *chosen (may be NULL).  The reference has no
  * autotuner (its dispatch sizes are fixed in the task graph, src/rigid_body_manager.cpp:1284-1427). */
 bb_status bb_autotune(void* world, float dt, uint32_t substeps, uint32_t trial_steps, bb_solver_params* chosen);
 
