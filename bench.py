@@ -189,9 +189,11 @@ def peaks() -> dict:
 
 
 def solver_bytes(st: dict, n: int, args) -> float:
-    """Algorithmic HBM bytes of one solver launch (one substep), SoA float4 model: body
-    state 64 B, props 48 B, contact row 64 B, manifold header 32 B.  PGS: the manifolds and
-    contacts the colour sweeps solve (those with an awake body); AVBD: all of them."""
+    """Algorithmic HBM bytes of one solver launch (one substep), by a fixed model that does not follow
+    the kernels' own layout: SoA float4 arrays, body state 64 B, props 48 B, contact row 64 B,
+    manifold header 32 B.  PGS: the manifolds and contacts the colour sweeps solve (those with an
+    awake body); AVBD: all of them.  (The PGS_SOFT sweeps read 40 and write 16 bytes per contact,
+    read 216 per item and write 64 of body velocities, from L2 where it holds them.)"""
     if args.solver == "pgs":
         M, K = st["solved_manifolds"], st["solved_contacts"]
         it = pgs_iterations(args)
@@ -309,7 +311,7 @@ def kernel_roof(kernel: str, bytes_total: float, ms_total: float, launches: int,
             "ms_per_launch": ms_total / max(launches, 1), "launches": launches, "model": model}
 
 
-def profiled_window(bb, args, sc, local_rank: int, first: int, steps: int, peak_gbs: float, traffic=None) -> dict:
+def profiled_window(bb, args, sc, local_rank: int, first: int, steps: int, peak_gbs: float) -> dict:
     """A second world with the same deterministic history, profiled over the timed steps:
     per-stage CUDA-event times (a substep run stage by stage with events between) and the
     rooflines of the solver, the sort and the refit from their own event times and the
@@ -334,11 +336,14 @@ def profiled_window(bb, args, sc, local_rank: int, first: int, steps: int, peak_
     w.close()
     sort_b, refit_b = 68.0 * n * front_runs, 52.0 * n * front_runs
     subs = steps * SUBSTEPS
-    solver_name = "k_pgs_soft" if args.solver == "pgs" else "AVBD kernels"
+    pgs = args.solver == "pgs"
+    solver_name = "k_pgs_soft" if pgs else "AVBD kernels"
+    solver_model = ("fixed model, PGS_SOFT: pre-step 64K + 224M, each of 2I sweeps 64K + 128M, integrate 128N bytes "
+                    "(K contacts, M manifolds solved this substep)" if pgs else
+                    "fixed model, AVBD: 384N, each of 19 sweeps 64N + 64M + 128K, each of 4 dual steps 32M + 76K bytes")
     roofs = {
-        "solve": kernel_roof(f"solve ({solver_name})", solve_b, stages.get("solve", 0.0), subs, peak_gbs, traffic,
-                             "PGS_SOFT: pre-step 64K + 224M, each of 2I sweeps 64K + 128M, integrate 128N bytes "
-                             "(K contacts, M manifolds solved this substep)"),
+        "solve": kernel_roof(f"solve ({solver_name})", solve_b, stages.get("solve", 0.0), subs, peak_gbs, None,
+                             solver_model),
         "sort": kernel_roof("sort (k_sort_hist + 4x k_onesweep)", sort_b, stages.get("sort", 0.0), max(front_runs, 1),
                             peak_gbs, None, "68 B per body: histogram read 4 B + 4 passes x 16 B"),
         "refit": kernel_roof("refit (k_refit, node records fused)", refit_b, stages.get("refit", 0.0),
